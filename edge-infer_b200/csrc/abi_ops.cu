@@ -108,7 +108,7 @@ namespace {
 void run_prompt_operator(const ei_context* ctx, bool awq, GemmParams p, void* scratch, size_t scratch_bytes,
                          cudaStream_t stream) {
   const int ksplit = (scratch && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0)
-                         ? prompt_gemm_ksplit(p.M, p.N, p.K, ctx->multiprocessors, scratch_bytes) : 1;
+                         ? prompt_gemm_ksplit(awq, p.M, p.N, p.K, true, ctx->multiprocessors, scratch_bytes) : 1;
   if (ksplit < 2) {
     launch_prompt_gemm(awq, p, stream, false);
     return;

@@ -1484,7 +1484,7 @@ void enqueue_layered_segment(ei_session& s, int rows, size_t context) {
   enqueue_embed<bf16>(s, b, token);
 
   const auto sums = [&](const PreparedLinear& w, const bf16* x, float* partial) {
-    const int ksplit = prompt_gemm_ksplit(rows, w.out, w.in, model.multiprocessors, ws.partial_bytes);
+    const int ksplit = prompt_gemm_ksplit(w.quantized, rows, w.out, w.in, false, model.multiprocessors, ws.partial_bytes);
     run_prompt_linear(s, w, x, rows, nullptr, pdl, ksplit, 0, partial);
     return ksplit;
   };

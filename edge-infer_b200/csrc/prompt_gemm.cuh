@@ -5,23 +5,38 @@
 // kernels (one pass over the weights per 16 rows) are the wrong tool: here every weight is dequantised once per
 // 256 tokens and multiplied on tcgen05.
 //
-// A block owns a tile of 256 output features and up to 256 tokens (two token tiles of 128, the M of one MMA), and
-// walks K in blocks of 64 inputs through a ring of stages:
-//   * one thread (warp 8) issues the TMA copies of a stage: the activations of both token tiles as
-//     [128 tokens][64 inputs] BF16 boxes with the 128-byte swizzle (the K-major operand layout of tcgen05.mma),
-//     and the weights - BF16 weights as one [256 features][64 inputs] swizzled box, int4 weights as a raw
-//     [256 rows][32 bytes] box;
-//   * for int4, warps 0-7 turn the raw box into the BF16 K-major swizzled operand in shared memory with the
-//     exact dequantisation of the small-M kernels (dequant_pair: round_bf16((w - z) * scale)), fence the writes
-//     towards the asynchronous proxy and arrive on the stage's `ready` barrier;
-//   * one thread (warp 9) issues, per stage and token tile, four tcgen05.mma (M 128, N 256, K 16) that
-//     accumulate in tensor memory - 2 token tiles x 256 FP32 columns = all 512 columns - and commits the stage's
-//     `empty` barrier, which hands the stage back to the copy thread;
-//   * after the last K block warps 0-7 read the accumulators with tcgen05.ld (warp w: lanes 32 (w % 4) ..., token
-//     tile w / 4), add the bias in FP32, round once to BF16 and store whole output rows through shared memory -
-//     or, for a projection whose sum the
-//     residual + norm kernel finishes, store FP32 partial sums, K split over blockIdx.z so that few token tiles
-//     still fill the SMs.
+// The features are the M of the MMA (128 per tile, one or two tiles per block) and the tokens its N: a block owns
+// feature_tiles x 128 features (int4: 128) and token_tiles x columns tokens (columns a multiple of 16, at most 256; at
+// most 512 accumulator columns in all). So a tile is cut to the rows there are - 333 tokens are two tiles of 176, 320 are
+// one pass over the weights with two tiles of 160 - where a tile of 128 tokens as M would leave up to 127 of them empty
+// and dequantise the weights once more. The host chooses the shape from the cost of a K block (prompt_choice).
+// A block walks K in blocks of 64 inputs through rings of their own for activations, weights and, int4, packed weights (a
+// ring's depth has to hide its own latency only: a copy's for activations and packed weights, the way from a free operand
+// buffer through conversion and MMA for the dequantised ones):
+//   * two threads (warps 16 and 19) issue the TMA copies, one those of the weights and one those of the activations: the
+//     activations as [columns tokens][64 inputs] BF16 boxes with the 128-byte swizzle (the K-major operand layout of
+//     tcgen05.mma), BF16 weights as [128 features][64 inputs] swizzled boxes, int4 weights as raw [128 rows][32 bytes]
+//     boxes. The weights of the ring's first round are requested before the kernel waits for its predecessor, which does
+//     not write them;
+//   * for int4, teams of four of warps 0-15 turn the raw boxes into the BF16 K-major swizzled operand in shared memory,
+//     team j of w_stages every w_stages-th K block, with the exact dequantisation of the small-M kernels (dequant_pair:
+//     round_bf16((w - z) * scale)), fence the writes towards the asynchronous proxy and arrive on the K block's `ready`
+//     barrier;
+//   * one warp or, with more than one accumulator, two (warps 17 and 18) issue, per K block, feature tile and token
+//     tile, four tcgen05.mma (M 128, N columns, K 16) that accumulate in tensor memory, and commit the K block's `empty`
+//     barrier, which hands both operands' buffers back;
+//   * after the last K block warps 0-15 read the accumulators with tcgen05.ld (warp w: features 32 (w % 4) ..., every
+//     fourth group of 16 tokens from w / 4). A lane is a feature, so the bias is one register and a token's 32 features
+//     leave a warp as one 128-byte line of FP32 sums or, after an exchange between neighbouring lanes, as 64 bytes of
+//     BF16. For a projection whose sum the residual + norm kernel finishes the FP32 partial sums are stored, K split
+//     over blockIdx.z so that few tiles still fill the SMs.
+// What bounds it, by leaving parts out in copies of the kernel: the instruction chain of the thread that issues the MMAs,
+// then shared memory. With one lane walking the issuing loop a K block of a 128-feature tile took 575 (BF16) and 800 (int4)
+// cycles at any number of tokens; with warp-uniform descriptors, one barrier and one commit per K block it takes 380 and
+// 540-560 at up to 160 tokens, and above that what the copies in, the dequantised weights in and the MMAs' operands out
+// take at 128 bytes a cycle (1005-1050 of 1031 at 128 x 320). Measured, int4, per launch, first form (tiles of 128 tokens
+// as M, 256 features) -> this one: 37888 x 3584, 320 rows 105 -> 66 us; 24576 x 4096, 2048 rows 357 -> 297-312 us;
+// BF16: 4096 x 2048, 333 rows 15 -> 9.9 us.
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
 //
 // Every wait on an mbarrier is bounded. A role whose wait runs out raises a flag in shared memory that every
@@ -34,26 +49,35 @@
 
 namespace ei {
 
-constexpr int kPromptTokens = 128;     // tokens per token tile = M of one MMA
-constexpr int kPromptTokenTiles = 2;   // token tiles per block
-constexpr int kPromptFeatures = 256;   // output features per block = N of one MMA
+constexpr int kPromptFeatures = 128;   // features per feature tile = M of one MMA
+constexpr int kPromptMaxColumns = 256; // tokens per token tile = N of one MMA, at most
+constexpr int kPromptTmemColumns = 512;
 constexpr int kPromptBlockK = 64;      // inputs per stage: one 128-byte swizzle row of BF16
-constexpr int kPromptStages = 3;
-constexpr int kPromptWorkerWarps = 8;
-constexpr int kPromptThreads = (kPromptWorkerWarps + 2) * 32;
-constexpr int kPromptTileBytes = kPromptTokens * kPromptBlockK * 2;                 // 16 KiB per token tile
-constexpr int kPromptWeightBytes = kPromptFeatures * kPromptBlockK * 2;             // 32 KiB BF16 operand
-constexpr int kPromptRawBytes = kPromptFeatures * (kPromptBlockK / 2);              // 8 KiB of int4
-constexpr int kPromptStageBytes = kPromptTokenTiles * kPromptTileBytes + kPromptWeightBytes + kPromptRawBytes;
-constexpr size_t kPromptSharedBytes = size_t(kPromptStages) * kPromptStageBytes + 1024 /* alignment */ + 256;
+constexpr int kPromptMaxStages = 8;
+constexpr int kPromptWorkerWarps = 16;
+constexpr int kPromptTeamWarps = 4;    // int4: a team of warps dequantises a K block of the one feature tile
+constexpr int kPromptThreads = (kPromptWorkerWarps + 4) * 32;
+constexpr int kPromptWeightBytes = kPromptFeatures * kPromptBlockK * 2;             // 16 KiB BF16 operand per feature tile
+constexpr int kPromptRawBytes = kPromptFeatures * (kPromptBlockK / 2);              // 4 KiB of int4 per feature tile
+constexpr size_t kPromptSharedExtra = 1024 /* alignment */ + 512;
+
+// Bytes of the rings: activations, weight operands, packed int4 weights (every stage a multiple of 1024).
+__host__ __device__ inline int prompt_ring_bytes(const PromptTile& t) {
+  return t.x_stages * t.token_tiles * t.columns * kPromptBlockK * 2 +
+         t.feature_tiles * (t.w_stages * kPromptWeightBytes + t.raw_stages * kPromptRawBytes);
+}
 
 struct PromptMaps {
-  CUtensorMap x;        // bf16 [T][K], box [128][64], 128-byte swizzle
-  CUtensorMap weights;  // int4: u32 [N][K/8], box [256][8]; BF16: bf16 [N][K], box [256][64], 128-byte swizzle
+  CUtensorMap x;        // bf16 [T][K], box [columns][64], 128-byte swizzle
+  CUtensorMap weights;  // int4: u32 [N][K/8], box [128][8]; BF16: bf16 [N][K], box [128][64], 128-byte swizzle
 };
 
 struct PromptShared {
-  uint64_t full[kPromptStages], ready[kPromptStages], empty[kPromptStages], done;
+  // Both operands of a K block are there / have been read, in a ring as long as that of the activations: one wait and
+  // one commit per K block, because the warp that issues the MMAs is what bounds a small tile.
+  uint64_t ready[kPromptMaxStages], empty[kPromptMaxStages];
+  uint64_t raw_full[kPromptMaxStages], raw_empty[kPromptMaxStages];  // packed int4 weights
+  uint64_t done;
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -74,15 +98,18 @@ __device__ __forceinline__ void tcgen05_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_address(bar))
                : "memory");
 }
-// D[tmem_d] (+)= A[desc_a] * B[desc_b]^T, both operands K-major in shared memory, FP32 accumulation.
-__device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                             uint32_t accumulate) {
+// D[tmem_d] (+)= A * B^T, both operands K-major in shared memory, FP32 accumulation. The operands' descriptors are given
+// by their low words; the high word is the same for every K-major 128-byte-swizzled operand.
+__device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t desc_high,
+                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
       :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(desc_high), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tmem_load16(uint32_t address, float (&v)[16]) {
@@ -101,13 +128,14 @@ __device__ __forceinline__ void tmem_load16(uint32_t address, float (&v)[16]) {
 
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled operand: rows 128 bytes apart, groups of eight
 // rows 1024 bytes apart; bits [46,48) carry the descriptor version of this architecture, bits [61,64) the swizzle.
-__device__ __forceinline__ uint64_t umma_kmajor_sw128_desc(uint32_t shared_address) {
-  return uint64_t((shared_address & 0x3ffffu) >> 4) | (uint64_t(1) << 16) | (uint64_t(1024 >> 4) << 32) |
-         (uint64_t(1) << 46) | (uint64_t(2) << 61);
+__device__ __forceinline__ uint32_t umma_desc_low(uint32_t shared_address) {
+  return ((shared_address & 0x3ffffu) >> 4) | (1u << 16);
 }
-// Instruction descriptor: D FP32, A and B BF16, both K-major, N = 256, M = 128.
-constexpr uint32_t kPromptInstruction =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t(kPromptFeatures) >> 3) << 17) | ((uint32_t(kPromptTokens) >> 4) << 24);
+constexpr uint32_t kUmmaDescHigh = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);
+// Instruction descriptor: D FP32, A and B BF16, both K-major, M = 128, N = `columns`.
+__device__ __forceinline__ uint32_t prompt_instruction(int columns) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t(columns) >> 3) << 17) | ((uint32_t(kPromptFeatures) >> 4) << 24);
+}
 
 // Bounded wait that also gives up as soon as another role of the block has.
 __device__ __forceinline__ bool prompt_wait(PromptShared* sh, uint64_t* bar, uint32_t parity, uint32_t limit) {
@@ -119,6 +147,12 @@ __device__ __forceinline__ bool prompt_wait(PromptShared* sh, uint64_t* bar, uin
   sh->abort = 1;
   return false;
 }
+// 1 in one lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected;
+}
 __device__ __forceinline__ void mbarrier_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_address(bar)) : "memory");
 }
@@ -129,12 +163,12 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   extern __shared__ unsigned char prompt_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(prompt_smem_raw) + 1023) &
                                                          ~uintptr_t(1023));
-  PromptShared* sh = reinterpret_cast<PromptShared*>(smem + size_t(kPromptStages) * kPromptStageBytes);
+  const int columns = p.prompt.columns, block_tokens = p.prompt.token_tiles * columns;
+  PromptShared* sh = reinterpret_cast<PromptShared*>(smem + prompt_ring_bytes(p.prompt));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // p.prompt_tiles (1 or 2) token tiles per block: chosen on the host so that the grid's waves are well filled.
-  const int tiles_per_block = p.prompt_tiles == 1 ? 1 : kPromptTokenTiles;
-  const int n0 = blockIdx.x * kPromptFeatures, t0 = blockIdx.y * (kPromptTokens * tiles_per_block);
-  const int token_tiles = min(tiles_per_block, (p.M - t0 + kPromptTokens - 1) / kPromptTokens);
+  const int n0 = blockIdx.x * kPromptFeatures * p.prompt.feature_tiles, t0 = blockIdx.y * block_tokens;
+  const int feature_tiles = min(p.prompt.feature_tiles, (p.N - n0 + kPromptFeatures - 1) / kPromptFeatures);
+  const int token_tiles = min(p.prompt.token_tiles, (p.M - t0 + columns - 1) / columns);
   // K slice of this block (blockIdx.z of p.ksplit): whole quantisation groups, i.e. pairs of K blocks.
   const int slice = blockIdx.z;
   const int pairs_total = p.K / (2 * kPromptBlockK);
@@ -142,212 +176,259 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   const int kb_end = p.ksplit > 1 ? int((long long)(slice + 1) * pairs_total / p.ksplit) * 2 : p.K / kPromptBlockK;
   const int k_blocks = kb_end - kb_begin;
   const uint32_t limit = p.wait_limit ? p.wait_limit : kAwqWaitLimit;
+  const int issuers = min(2, p.prompt.feature_tiles * p.prompt.token_tiles);  // warps that issue MMAs
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPromptStages; ++s) {
-      mbarrier_init(&sh->full[s], 1);
-      mbarrier_init(&sh->ready[s], kPromptWorkerWarps);
-      mbarrier_init(&sh->empty[s], 1);
+    for (int s = 0; s < kPromptMaxStages; ++s) {
+      mbarrier_init(&sh->ready[s], kAwq ? 1 + kPromptTeamWarps : 2);
+      mbarrier_init(&sh->empty[s], issuers);
+      mbarrier_init(&sh->raw_full[s], 1);
+      mbarrier_init(&sh->raw_empty[s], kPromptTeamWarps);
     }
-    mbarrier_init(&sh->done, 1);
+    mbarrier_init(&sh->done, issuers);
     sh->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kPromptWorkerWarps + 1) tmem_alloc(&sh->tmem_base, 512);
+  if (warp == kPromptWorkerWarps + 1) tmem_alloc(&sh->tmem_base, kPromptTmemColumns);
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem = sh->tmem_base;
-  grid_dependency_wait();
-  grid_launch_dependents();
 
-  auto stage_base = [&](int s) { return smem + size_t(s) * kPromptStageBytes; };
-  constexpr int kWeightOffset = kPromptTokenTiles * kPromptTileBytes;
-  constexpr int kRawOffset = kWeightOffset + kPromptWeightBytes;
+  const int tile_bytes = columns * kPromptBlockK * 2;  // activations of one token tile
+  const int x_bytes = p.prompt.token_tiles * tile_bytes, w_bytes = p.prompt.feature_tiles * kPromptWeightBytes;
+  const int raw_bytes = p.prompt.feature_tiles * kPromptRawBytes;
+  unsigned char* const x_ring = smem;
+  unsigned char* const w_ring = x_ring + p.prompt.x_stages * x_bytes;
+  unsigned char* const raw_ring = w_ring + p.prompt.w_stages * w_bytes;
 
-  if (warp == kPromptWorkerWarps) {
-    // ---- copy thread ----
-    if (lane == 0) {
-      const uint32_t bytes = uint32_t(token_tiles) * kPromptTileBytes + (kAwq ? kPromptRawBytes : kPromptWeightBytes);
-      int issued = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        const int s = kb % kPromptStages;
-        if (kb >= kPromptStages && !prompt_wait(sh, &sh->empty[s], ((kb / kPromptStages) - 1) & 1, limit)) break;
-        mbarrier_expect_tx(&sh->full[s], bytes + (kb == 0 ? p.fault_tx : 0u));
-        unsigned char* base = stage_base(s);
+  if (warp == kPromptWorkerWarps || warp == kPromptWorkerWarps + 3) {
+    // ---- copy threads: one for the weights, one for the activations ----
+    const bool weights = warp == kPromptWorkerWarps;
+    const int stages = !weights ? p.prompt.x_stages : kAwq ? p.prompt.raw_stages : p.prompt.w_stages;
+    uint64_t* const full = weights && kAwq ? sh->raw_full : sh->ready;
+    uint64_t* const empty = weights && kAwq ? sh->raw_empty : sh->empty;
+    auto request = [&](int kb, int s) {
+      if (weights) {
+        mbarrier_expect_tx(&full[s], uint32_t(feature_tiles) * (kAwq ? kPromptRawBytes : kPromptWeightBytes) +
+                                         (kb == 0 ? p.fault_tx : 0u));
+        for (int f = 0; f < feature_tiles; ++f) {
+          if (kAwq)
+            tma_load_2d(raw_ring + s * raw_bytes + f * kPromptRawBytes, &maps.weights, (kb_begin + kb) * (kPromptBlockK / 8),
+                        n0 + f * kPromptFeatures, &full[s]);
+          else
+            tma_load_2d(w_ring + s * w_bytes + f * kPromptWeightBytes, &maps.weights, (kb_begin + kb) * kPromptBlockK,
+                        n0 + f * kPromptFeatures, &full[s]);
+        }
+      } else {
+        mbarrier_expect_tx(&full[s], uint32_t(token_tiles * tile_bytes));
         for (int mt = 0; mt < token_tiles; ++mt)
-          tma_load_2d(base + mt * kPromptTileBytes, &maps.x, (kb_begin + kb) * kPromptBlockK, t0 + mt * kPromptTokens,
-                      &sh->full[s]);
-        if (kAwq)
-          tma_load_2d(base + kRawOffset, &maps.weights, (kb_begin + kb) * (kPromptBlockK / 8), n0, &sh->full[s]);
-        else
-          tma_load_2d(base + kWeightOffset, &maps.weights, (kb_begin + kb) * kPromptBlockK, n0, &sh->full[s]);
+          tma_load_2d(x_ring + s * x_bytes + mt * tile_bytes, &maps.x, (kb_begin + kb) * kPromptBlockK, t0 + mt * columns,
+                      &full[s]);
+      }
+    };
+    const int early = min(stages, k_blocks);
+    if (weights && lane == 0)
+      for (int kb = 0; kb < early; ++kb) request(kb, kb);
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (lane == 0) {
+      if (!weights)
+        for (int kb = 0; kb < early; ++kb) request(kb, kb);
+      int issued = early, slot = 0;
+      uint32_t parity = 0;
+      for (int kb = early; kb < k_blocks; ++kb) {
+        if (!prompt_wait(sh, &empty[slot], parity, limit)) break;
+        request(kb, slot);
         issued = kb + 1;
+        if (++slot == stages) {
+          slot = 0;
+          parity ^= 1;
+        }
       }
       if (sh->abort) {
         // Copies still in flight write into this block's shared memory: wait for them (bounded) before leaving.
-        // The copy of K block 0 carries the test hook's unmet expectation and is known never to complete.
-        for (int kb = max(p.fault_tx ? 1 : 0, issued - kPromptStages); kb < issued; ++kb) {
-          const int s = kb % kPromptStages;
+        // The weights of K block 0 carry the test hook's unmet expectation and are known never to complete.
+        for (int kb = max(p.fault_tx ? 1 : 0, issued - stages); kb < issued; ++kb) {
+          const int s = kb % stages;
           for (uint32_t polls = 0; polls < limit; ++polls)
-            if (mbarrier_try_wait(&sh->full[s], (kb / kPromptStages) & 1)) break;
+            if (mbarrier_try_wait(&full[s], (kb / stages) & 1)) break;
         }
       }
     }
-  } else if (warp == kPromptWorkerWarps + 1) {
-    // ---- MMA thread ----
-    if (lane == 0) {
+  } else if (warp > kPromptWorkerWarps) {
+    // ---- MMA warps: warp i issues for the accumulators i, i + issuers, ... (feature tile major). The whole warp walks
+    // the loop and one elected lane issues, so that descriptors and counters are warp-uniform values. ----
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int mine = __shfl_sync(0xffffffffu, warp - (kPromptWorkerWarps + 1), 0);
+    if (mine < issuers) {
       bool issued = false;
+      const uint32_t leader = elect_one();
+      const uint32_t instruction = prompt_instruction(columns);
+      const int live = feature_tiles * token_tiles, second = mine + issuers;  // at most two accumulators per warp
+      const int f0 = mine / token_tiles, m0 = mine - f0 * token_tiles, f1 = second / token_tiles, m1 = second - f1 * token_tiles;
+      const uint32_t a0 = umma_desc_low(smem_address(w_ring) + f0 * kPromptWeightBytes);
+      const uint32_t b0 = umma_desc_low(smem_address(x_ring) + m0 * tile_bytes);
+      const uint32_t a1 = umma_desc_low(smem_address(w_ring) + f1 * kPromptWeightBytes);
+      const uint32_t b1 = umma_desc_low(smem_address(x_ring) + m1 * tile_bytes);
+      const uint32_t d0 = tmem + f0 * block_tokens + m0 * columns, d1 = tmem + f1 * block_tokens + m1 * columns;
+      const uint32_t w_step = uint32_t(w_bytes) >> 4, x_step = uint32_t(x_bytes) >> 4;
+      int w_slot = 0, slot = 0;
+      uint32_t parity = 0, w_at = 0, x_at = 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
-        const int s = kb % kPromptStages;
-        if (!prompt_wait(sh, kAwq ? &sh->ready[s] : &sh->full[s], (kb / kPromptStages) & 1, limit)) break;
+        if (!__all_sync(0xffffffffu, prompt_wait(sh, &sh->ready[slot], parity, limit))) break;
         tcgen05_fence_after();
-        const uint32_t base = smem_address(stage_base(s));
-        const uint64_t b_desc = umma_kmajor_sw128_desc(base + kWeightOffset);
-        for (int mt = 0; mt < token_tiles; ++mt) {
-          const uint64_t a_desc = umma_kmajor_sw128_desc(base + mt * kPromptTileBytes);
+        if (leader) {
+          if (mine < live) {
 #pragma unroll
-          for (int j = 0; j < kPromptBlockK / 16; ++j)  // 16 inputs = 32 bytes further along the swizzled row
-            umma_bf16_ss(tmem + mt * kPromptFeatures, a_desc + uint64_t(j * 2), b_desc + uint64_t(j * 2),
-                         kPromptInstruction, (kb > 0 || j > 0) ? 1u : 0u);
+            for (int j = 0; j < kPromptBlockK / 16; ++j)  // 16 inputs = 32 bytes further along the swizzled row
+              umma_bf16_ss(d0, a0 + w_at + j * 2, b0 + x_at + j * 2, kUmmaDescHigh, instruction, j > 0 ? 1u : uint32_t(kb));
+          }
+          if (second < live) {
+#pragma unroll
+            for (int j = 0; j < kPromptBlockK / 16; ++j)
+              umma_bf16_ss(d1, a1 + w_at + j * 2, b1 + x_at + j * 2, kUmmaDescHigh, instruction, j > 0 ? 1u : uint32_t(kb));
+          }
+          tcgen05_commit(&sh->empty[slot]);
         }
-        tcgen05_commit(&sh->empty[s]);
         issued = true;
+        w_at += w_step;
+        x_at += x_step;
+        if (++w_slot == p.prompt.w_stages) {
+          w_slot = 0;
+          w_at = 0;
+        }
+        if (++slot == p.prompt.x_stages) {
+          slot = 0;
+          x_at = 0;
+          parity ^= 1;
+        }
       }
-      tcgen05_commit(&sh->done);  // arrives when every MMA issued so far has completed
-      if (sh->abort && issued) {
-        for (uint32_t polls = 0; polls < limit; ++polls)
-          if (mbarrier_try_wait(&sh->done, 0)) break;
+      if (leader) {
+        tcgen05_commit(&sh->done);  // arrives when every MMA issued so far has completed
+        if (sh->abort && issued) {
+          for (uint32_t polls = 0; polls < limit; ++polls)
+            if (mbarrier_try_wait(&sh->done, 0)) break;
+        }
       }
     }
   } else {
     // ---- workers: dequantisation (int4 only), then the epilogue ----
     if (kAwq) {
-      // Thread t converts (row t / 2, half t % 2) and (row 128 + t / 2, half t % 2) of every stage: a half is 32
-      // inputs = 16 raw bytes = four 16-byte chunks of the operand row.
-      const int half = threadIdx.x & 1;
-      int rows[2], live_rows[2];
-      rows[0] = threadIdx.x >> 1;
-      rows[1] = 128 + rows[0];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) live_rows[i] = min(n0 + rows[i], p.N - 1);
-      // Scales and zero points of a group are requested one group (two K blocks) before they are used.
-      uint32_t scale2[2] = {0, 0}, zero_word[2] = {0, 0}, scale_next[2], zero_next[2];
-      const int group_begin = kb_begin >> 1, group_end = kb_end >> 1;
-      auto request = [&](int g) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          scale_next[i] = uint32_t(__bfloat16_as_ushort(p.scales[size_t(live_rows[i]) * p.padded_groups + g])) * 0x10001u;
-          zero_next[i] = ((g & 7) == 0 || g == group_begin) ? uint32_t(p.zeros[size_t(live_rows[i]) * p.zero_stride + (g >> 3)]) : zero_word[i];
-        }
+      // Team j of w_stages converts K blocks j, j + w_stages, ... into operand buffer j, from the raw buffers j, j +
+      // w_stages, ...: every buffer belongs to one team, so no team can miss a phase of its barriers. A thread owns one
+      // row: 64 inputs = 32 raw bytes = eight 16-byte chunks of the operand row.
+      const int teams = p.prompt.w_stages, team = warp / kPromptTeamWarps, row = threadIdx.x & (kPromptFeatures - 1);
+      const int live_row = min(n0 + row, p.N - 1);
+      const bf16* scales = p.scales + size_t(live_row) * p.padded_groups;
+      const int32_t* zeros = p.zeros + size_t(live_row) * p.zero_stride;
+      // Scales and zero points are requested one of the team's K blocks before they are used.
+      uint32_t scale_next = 0, zero_next = 0, zero_shift = 0;
+      auto request = [&](int kb) {
+        const int g = (kb_begin + kb) >> 1;  // 128 inputs per group, 64 per K block
+        scale_next = __bfloat16_as_ushort(scales[g]);
+        zero_next = uint32_t(zeros[g >> 3]);
+        zero_shift = (g & 7) * 4;
       };
-      request(group_begin);
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        const int s = kb % kPromptStages;
-        const int grp = (kb_begin + kb) >> 1;  // 128 inputs per group, 64 per K block
-        if ((kb & 1) == 0) {
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            scale2[i] = scale_next[i];
-            zero_word[i] = zero_next[i];
+      const int end = team < teams ? k_blocks : 0;
+      if (team < end) request(team);
+      unsigned char* const operand = w_ring + team * w_bytes + row * 128;
+      // Rows 4-7 of eight read their halves in the other order: the eight lanes of a load hit distinct banks.
+      const unsigned char* const raw_row = raw_ring + row * 32;
+      const int first_half = (row & 4) * 4;
+      // K block kb takes the operand buffer that K block kb - teams leaves; the MMAs complete in order and the ring of
+      // `empty` is at least as long as that of the operands, so the phase waited for is the next one to complete.
+      int raw_slot = team, ready_slot = team, left_slot = team;
+      uint32_t raw_parity = 0, left_parity = 0;
+      for (int kb = team; kb < end; kb += teams) {
+        const uint32_t scale2 = scale_next * 0x10001u, zero2 = (0x4300u | ((zero_next >> zero_shift) & 15u)) * 0x10001u;
+        if (kb + teams < end) request(kb + teams);
+        // The loop is left by whole warps: the barriers and the votes below are warp-wide.
+        if (!__all_sync(0xffffffffu, prompt_wait(sh, &sh->raw_full[raw_slot], raw_parity, limit))) break;
+        const uint4 raw0 = *reinterpret_cast<const uint4*>(raw_row + raw_slot * raw_bytes + first_half);
+        const uint4 raw1 = *reinterpret_cast<const uint4*>(raw_row + raw_slot * raw_bytes + 16 - first_half);
+        const uint32_t words[8] = {raw0.x, raw0.y, raw0.z, raw0.w, raw1.x, raw1.y, raw1.z, raw1.w};
+        if (kb != team) {  // the buffer is fresh in the team's first round
+          if (!__all_sync(0xffffffffu, prompt_wait(sh, &sh->empty[left_slot], left_parity, limit))) break;
+          left_slot += teams;
+          if (left_slot >= p.prompt.x_stages) {
+            left_slot -= p.prompt.x_stages;
+            left_parity ^= 1;
           }
-          if (grp + 1 < group_end) request(grp + 1);
         }
-        // The loop is left by whole warps: the barrier and the vote below are warp-wide.
-        const bool arrived = prompt_wait(sh, &sh->full[s], (kb / kPromptStages) & 1, limit);
-        if (!__all_sync(0xffffffffu, arrived)) break;
-        unsigned char* base = stage_base(s);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int row = rows[i];
-          const uint4 raw = *reinterpret_cast<const uint4*>(base + kRawOffset + row * 32 + half * 16);
-          const uint32_t zero2 = (0x4300u | ((zero_word[i] >> ((grp & 7) * 4)) & 15u)) * 0x10001u;
-          const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            // dequant_pair gives (k, k + 4) pairs; the operand wants the eight inputs of a word in order.
-            const uint32_t p0 = dequant_pair(words[w], zero2, scale2[i]);
-            const uint32_t p1 = dequant_pair(words[w] >> 4, zero2, scale2[i]);
-            const uint32_t p2 = dequant_pair(words[w] >> 8, zero2, scale2[i]);
-            const uint32_t p3 = dequant_pair(words[w] >> 12, zero2, scale2[i]);
-            uint4 o;
-            o.x = __byte_perm(p0, p1, 0x5410);
-            o.y = __byte_perm(p2, p3, 0x5410);
-            o.z = __byte_perm(p0, p1, 0x7632);
-            o.w = __byte_perm(p2, p3, 0x7632);
-            const int chunk = (half * 4 + w) ^ (row & 7);
-            *reinterpret_cast<uint4*>(base + kWeightOffset + row * 128 + chunk * 16) = o;
-          }
+        for (int w = 0; w < 8; ++w) {
+          // dequant_pair gives (k, k + 4) pairs; the operand wants the eight inputs of a word in order.
+          const uint32_t p0 = dequant_pair(words[w], zero2, scale2);
+          const uint32_t p1 = dequant_pair(words[w] >> 4, zero2, scale2);
+          const uint32_t p2 = dequant_pair(words[w] >> 8, zero2, scale2);
+          const uint32_t p3 = dequant_pair(words[w] >> 12, zero2, scale2);
+          uint4 o;
+          o.x = __byte_perm(p0, p1, 0x5410);
+          o.y = __byte_perm(p2, p3, 0x5410);
+          o.z = __byte_perm(p0, p1, 0x7632);
+          o.w = __byte_perm(p2, p3, 0x7632);
+          *reinterpret_cast<uint4*>(operand + ((w ^ (row & 4) ^ (row & 7)) << 4)) = o;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbarrier_arrive(&sh->ready[s]);
+        if (lane == 0) {
+          mbarrier_arrive(&sh->ready[ready_slot]);
+          mbarrier_arrive(&sh->raw_empty[raw_slot]);
+        }
+        ready_slot += teams;
+        if (ready_slot >= p.prompt.x_stages) ready_slot -= p.prompt.x_stages;
+        raw_slot += teams;
+        if (raw_slot >= p.prompt.raw_stages) {
+          raw_slot = team;
+          raw_parity ^= 1;
+        }
       }
     }
+    // The dequantisation above reads weights only; the outputs below may be read by the predecessor.
+    grid_dependency_wait();
+    grid_launch_dependents();
     // ---- epilogue ----
     const bool complete = __all_sync(0xffffffffu, prompt_wait(sh, &sh->done, 0, limit) && !sh->abort);
     tcgen05_fence_after();
-    const int quarter = warp & 3, mt = warp >> 2;
-    if (complete && mt < token_tiles) {
-      // The accumulators come out of tensor memory one token per lane, which would make every store of a warp hit
-      // 32 different output rows. They go through shared memory instead (the ring's stages are free by now; a
-      // padded row pitch keeps both directions conflict-free), 128 columns at a time, and leave as whole rows:
-      // sixteen lanes write 256 contiguous bytes of a BF16 row (thirty-two lanes 512 bytes of an FP32 one).
-      const bool partial = p.epilogue == kEpiPartial;
-      constexpr int kPitch = 528;  // bytes per staged row: 512 of FP32 (or 256 of BF16) plus 16
-      unsigned char* staged = smem + size_t(warp) * 32 * kPitch;
-      const int first_token = t0 + mt * kPromptTokens + quarter * 32;
+    const int quarter = warp & 3;
+    const int tokens = min(token_tiles * columns, p.M - t0);  // live ones of this block
+    constexpr int kEpilogueStep = kPromptWorkerWarps / 4 * 16;
+    if (complete) {
+      const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
+      const bool odd = lane & 1;
+      // Two neighbouring lanes (features) exchange one of two tokens' values, so that each stores a pair of features.
+      auto store_pairs = [&](const float (&v)[16], int token, int first_feature) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+          const uint32_t packed = odd ? pack_bf16(other, v[i + 1]) : pack_bf16(v[i], other);
+          const int mine = token + i + (odd ? 1 : 0);
+          if (mine < p.M && first_feature < p.N)
+            *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_feature) = packed;
+        }
+      };
+      for (int f = 0; f < feature_tiles; ++f) {
+        const int feature = n0 + f * kPromptFeatures + quarter * 32 + lane;
+        const float bias = p.bias && feature < p.N ? __bfloat162float(p.bias[feature]) : 0.0f;
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        if (n0 + half * 128 >= p.N) break;  // block-uniform
-#pragma unroll 1
-        for (int cb = 0; cb < 8; ++cb) {
+        for (int c = (warp >> 2) * 16; c < tokens; c += kEpilogueStep) {
           float v[16];
-          tmem_load16(tmem + (uint32_t(quarter * 32) << 16) + mt * kPromptFeatures + half * 128 + cb * 16, v);
-          if (partial) {
+          tmem_load16(lane_base + f * block_tokens + c, v);
+          if (p.epilogue == kEpiPartial) {
+            if (feature < p.N) {
+              float* dst = p.partial + (size_t(slice) * p.M + t0 + c) * p.N + feature;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              *reinterpret_cast<float4*>(staged + lane * kPitch + cb * 64 + i * 16) =
-                  make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          } else {
-            uint32_t packed[8];
-            const int column = n0 + half * 128 + cb * 16;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float a = v[2 * i], b = v[2 * i + 1];
-              if (p.bias && column + 2 * i + 1 < p.N) {
-                a += __bfloat162float(p.bias[column + 2 * i]);
-                b += __bfloat162float(p.bias[column + 2 * i + 1]);
-              }
-              packed[i] = pack_bf16(activated_value(p.activation, a), activated_value(p.activation, b));
+              for (int i = 0; i < 16; ++i)
+                if (t0 + c + i < p.M) dst[size_t(i) * p.N] = v[i];
             }
-            *reinterpret_cast<uint4*>(staged + lane * kPitch + cb * 32) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            *reinterpret_cast<uint4*>(staged + lane * kPitch + cb * 32 + 16) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = activated_value(p.activation, v[i] + bias);
+            store_pairs(v, t0 + c, feature & ~1);
           }
         }
-        __syncwarp();
-        if (partial) {
-          // One staged row (128 floats) per instruction.
-          const int column = n0 + half * 128 + lane * 4;
-#pragma unroll 4
-          for (int r = 0; r < 32; ++r) {
-            const int token = first_token + r;
-            if (token < p.M && column < p.N)
-              *reinterpret_cast<float4*>(p.partial + (size_t(slice) * p.M + token) * p.N + column) =
-                  *reinterpret_cast<const float4*>(staged + r * kPitch + lane * 16);
-          }
-        } else {
-          // Two staged rows (128 BF16 values each) per instruction.
-          const int column = n0 + half * 128 + (lane & 15) * 8;
-#pragma unroll 4
-          for (int r = lane >> 4; r < 32; r += 2) {
-            const int token = first_token + r;
-            if (token < p.M && column < p.N)
-              *reinterpret_cast<uint4*>(p.out + size_t(token) * p.out_stride + column) =
-                  *reinterpret_cast<const uint4*>(staged + r * kPitch + (lane & 15) * 16);
-          }
-        }
-        __syncwarp();
       }
     }
   }
@@ -356,7 +437,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   tcgen05_fence_after();
   if (warp == kPromptWorkerWarps + 1) {
     __syncwarp();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, kPromptTmemColumns);
   }
   if (threadIdx.x == 0 && sh->abort && p.status) atomicOr(p.status, 4);
 }

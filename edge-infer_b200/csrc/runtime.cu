@@ -334,7 +334,7 @@ void run_prompt_linear_store(ei_session& s, const PreparedLinear& w, const bf16*
                              int x_stride) {
   ei_model& m = *s.model;
   auto& ws = m.prompt;
-  const int ksplit = w.out % 4 == 0 ? prompt_gemm_ksplit(rows, w.out, w.in, m.multiprocessors, ws.partial_bytes) : 1;
+  const int ksplit = w.out % 4 == 0 ? prompt_gemm_ksplit(w.quantized, rows, w.out, w.in, true, m.multiprocessors, ws.partial_bytes) : 1;
   if (ksplit < 2) {
     run_prompt_linear(s, w, x, rows, out, pdl, 0, x_stride);
     return;
@@ -520,7 +520,7 @@ void run_prompt_projection_residual_norm(ei_session& s, const PreparedLinear& w,
   auto& ws = m.prompt;
   const auto& c = m.config;
   if (w.out % 4 == 0 && size_t(rows) * w.out * sizeof(float) <= ws.partial_bytes) {
-    const int ksplit = prompt_gemm_ksplit(rows, w.out, w.in, m.multiprocessors, ws.partial_bytes);
+    const int ksplit = prompt_gemm_ksplit(w.quantized, rows, w.out, w.in, false, m.multiprocessors, ws.partial_bytes);
     run_prompt_linear(s, w, x, rows, nullptr, pdl, ksplit);
     ResidualNormParams p{};
     p.partial = ws.partial;

@@ -45,6 +45,13 @@ enum Activation : int {
   kActReluSquared = 1   // max(sum + bias, 0)^2, on the FP32 sum
 };
 
+// Shape of a prompt GEMM block (prompt_gemm.cuh): feature tiles of 128, token tiles of `columns` (a multiple of 16).
+struct PromptTile {
+  int feature_tiles, token_tiles, columns;
+  int x_stages, w_stages;  // K blocks of activations and of BF16 weights in the rings (x_stages >= w_stages)
+  int raw_stages;          // int4: K blocks of packed weights; a multiple of w_stages
+};
+
 struct GemmParams {
   const bf16* x;          // [M, K], row stride x_stride
   int x_stride;
@@ -68,7 +75,7 @@ struct GemmParams {
   int* best_index;        //             [grid, 16]
   int* status;            // optional device word; bit 2 is set if a bounded wait on a bulk copy gave up
   uint32_t wait_limit;    // polls before a bounded wait gives up (0: the kernel's default)
-  int prompt_tiles;       // prompt GEMM only: token tiles of 128 rows per block (0: chosen by the launch function)
+  PromptTile prompt;      // prompt GEMM only: filled in by its launch function
   uint32_t fault_tx;      // test hook: bytes the first weight copy is expected to deliver beyond what it does,
                           // so that the bounded waits run out (0 in production)
 };
@@ -419,11 +426,11 @@ bool prompt_gemm_eligible(bool awq, int group_size, int N, int K, const void* x,
                           int out_stride);
 // epilogue kEpiStore: out[T, N] = x[T, K] * W^T (+ bias), rounded once to BF16. kEpiPartial: FP32 partial sums
 // partial[ksplit][T][N] without bias, K split over ksplit blocks (whole groups of 128 inputs each).
-// Uses p.x, x_stride, M (= T), K, N, the weight fields of its kind, bias, out, out_stride, epilogue, ksplit,
+// Uses p.x, x_stride, M (= T), K, N, the weight fields of its kind, bias, out, out_stride, epilogue, activation, ksplit,
 // partial, status, wait_limit, fault_tx.
-int prompt_gemm_ksplit(int rows, int N, int K, int multiprocessors, size_t partial_bytes);
-// Token tiles per block (1 or 2) that fill the grid's waves best for this shape.
-int prompt_gemm_tiles(int rows, int N, int multiprocessors);
+// K slices worth using within the room of the partial buffer. `store`: the sums become a BF16 result through one more
+// kernel (1: no split, store directly); otherwise the caller finishes FP32 sums in any case.
+int prompt_gemm_ksplit(bool awq, int rows, int N, int K, bool store, int multiprocessors, size_t partial_bytes);
 void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool pdl);
 
 
