@@ -47,8 +47,9 @@ def test_awq_tiles(cuda, package, rows, nk):
     w = torch.from_numpy(np.ascontiguousarray(syn.awq_dequantize(q, s, z, k))).cuda().to(torch.bfloat16)
     gen = torch.Generator(device="cuda").manual_seed(rows * 17 + n)
     x = torch.randn((rows, k), device="cuda", generator=gen).to(torch.bfloat16)
-    weight = ops.prepare_awq(torch.from_numpy(q).cuda(), torch.from_numpy(s.view(np.int16)).cuda().view(torch.bfloat16),
-                             torch.from_numpy(z).cuda(), 128, k, None)
+    dq, dz = torch.from_numpy(q).cuda(), torch.from_numpy(z).cuda()   # the prepared weight borrows them
+    ds = torch.from_numpy(s.view(np.int16)).cuda().view(torch.bfloat16)
+    weight = ops.prepare_awq(dq, ds, dz, 128, k, None)
     ctx = ops.prepare_execution_context(0)
     scratch = torch.empty(ops.linear_scratch_bytes(rows, k, n), dtype=torch.uint8, device="cuda")
     for room in (None, scratch):
