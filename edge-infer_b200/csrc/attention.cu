@@ -481,7 +481,7 @@ void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool
   const unsigned sessions = q.slots ? unsigned(q.sessions) : 1u;
   launch(verify_attention_kernel<false>, dim3(q.kv_heads, q.max_splits, sessions), dim3(warps * 32), kAttentionShared,
          stream, pdl, q);
-  if (q.slots)
+  if (q.slots && !q.merge_blocks)
     launch(attention_merge_wide_kernel, dim3((q.rows * q.heads * q.sessions + 3) / 4), dim3(128), 0, stream, pdl, q);
   else
     launch(attention_merge_kernel, dim3(q.rows * q.heads, sessions), dim3(128), 0, stream, pdl, q);

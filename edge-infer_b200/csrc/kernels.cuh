@@ -152,6 +152,7 @@ struct AttentionParams {
   const SessionSlot* slots; // wide batch: one grid slice per session (`sessions` of them), `rows` query rows
   int sessions, layer;      // each; session j reads q + j * rows * q_stride, its own cache and context length,
   size_t scratch_stride;    // scratch + j * scratch_stride (floats), and writes out + j * rows * out_stride
+  bool merge_blocks;        // slots: merge with a block per (row, head), as for one session, instead of a warp
   // K / V tiles are fetched by TMA. A single session's maps are encoded by the launch function from k, v,
   // kv_stride, kv_heads and capacity; a wide batch passes one pair per session in device memory, built with
   // encode_kv_map over all layers of the session's cache (`layer` selects the slice).
@@ -191,12 +192,13 @@ void launch_finalize(const float* best_value, const int* best_index, int parts, 
 // Makes a draft session continue from where the target session stands: copies context length and pending token
 // and inherits a raised status. One thread.
 void launch_adopt_control(Control* mine, const Control* theirs, cudaStream_t stream);
-// Wide batch: per-row argmax partials laid out [row][parts] for any number of rows, then per session the final
-// argmax of its rows, acceptance against step_tokens and commit in its slot's control block.
+// Batches: per-row argmax partials laid out [row][parts] for any number of rows, then per session the final argmax of
+// its rows (part i of row r at i * part_stride + r * row_stride), acceptance against step_tokens and commit in its
+// slot's control block.
 void launch_argmax_partials_wide(const bf16* logits, size_t rows, size_t vocab, size_t row_stride, float* best_value,
                                  int* best_index, int parts, cudaStream_t stream, bool pdl);
-void launch_finalize_wide(const float* best_value, const int* best_index, int parts, int rows_per_session,
-                          int sessions, uint32_t* targets, const uint32_t* step_tokens, const SessionSlot* slots,
+void launch_finalize_wide(const float* best_value, const int* best_index, int parts, int part_stride, int row_stride,
+                          int rows_per_session, int sessions, uint32_t* targets, const uint32_t* step_tokens, const SessionSlot* slots,
                           cudaStream_t stream, bool pdl);
 
 // Acceptance only, from targets already chosen.

@@ -816,24 +816,23 @@ void enqueue_batch_step(ei_batch& batch, int rows) {
   const int qkv_width = (heads + 2 * kv_heads) * 128, kv_width = kv_heads * 128;
   const bool pdl = true;
 
-  for (int j = 0; j < count; ++j) {
-    ei_session& s = *batch.sessions[j];
-    EmbedParams e{};
-    e.tokens = lead.tokens + j * rows;
-    e.control = s.control;
-    e.step_tokens = lead.step_tokens + j * rows;
-    e.table = m.embedding;
-    e.vocab = int(c.vocab_size);
-    e.hidden = hidden;
-    e.rows = rows;
-    e.capacity = int(s.capacity);
-    e.norm_weight = m.layers[0].attention_norm;
-    e.eps = c.rms_norm_eps;
-    e.residual = lead.residual + size_t(j) * rows * hidden;
-    e.normed = lead.normed + size_t(j) * rows * hidden;
-    tick(lead);
-    launch_embed_norm(e, lead.stream, false);
-  }
+  // The per-session kernels are single launches that find a row's session in the slot array: at three sessions of five
+  // rows nine launches a layer (each some 2.3 us of a 90 us layer) become three.
+  EmbedParams e{};
+  e.tokens = lead.tokens;
+  e.step_tokens = lead.step_tokens;
+  e.table = m.embedding;
+  e.vocab = int(c.vocab_size);
+  e.hidden = hidden;
+  e.rows = total;
+  e.norm_weight = m.layers[0].attention_norm;
+  e.eps = c.rms_norm_eps;
+  e.residual = lead.residual;
+  e.normed = lead.normed;
+  e.slots = batch.slots;
+  e.rows_per_session = rows;
+  tick(lead);
+  launch_embed_norm(e, lead.stream, false);
   const size_t scratch_floats = attention_scratch_bytes(rows, heads, lead.capacity) / sizeof(float);
   for (size_t layer = 0; layer < m.layers.size(); ++layer) {
     const auto& L = m.layers[layer];
@@ -841,49 +840,45 @@ void enqueue_batch_step(ei_batch& batch, int rows) {
       run_linear(lead, L.qkv, lead.normed, total, kEpiStore, lead.qkv, qkv_width, pdl);
     else
       run_generic(lead, L.qkv, lead.normed, total, lead.qkv, pdl);
-    for (int j = 0; j < count; ++j) {
-      ei_session& s = *batch.sessions[j];
-      QkvParams q{};
-      q.qkv = lead.qkv + size_t(j) * rows * qkv_width;
-      q.rows = rows;
-      q.heads = heads;
-      q.kv_heads = kv_heads;
-      q.qkv_stride = qkv_width;
-      q.q_norm = c.qk_norm ? L.q_norm : nullptr;
-      q.k_norm = c.qk_norm ? L.k_norm : nullptr;
-      q.eps = c.rms_norm_eps;
-      q.rope_table = m.rope_table;
-      q.max_positions = int(c.max_position_embeddings);
-      q.control = s.control;
-      q.capacity = int(s.capacity);
-      q.k_cache = s.k_cache + layer * s.capacity * kv_width;
-      q.v_cache = s.v_cache + layer * s.capacity * kv_width;
-      tick(lead);
-      launch_qk_norm_rope_store(q, lead.stream, pdl);
-    }
-    for (int j = 0; j < count; ++j) {
-      ei_session& s = *batch.sessions[j];
-      AttentionParams a{};
-      a.q = lead.qkv + size_t(j) * rows * qkv_width;
-      a.q_stride = qkv_width;
-      a.k = s.k_cache + layer * s.capacity * kv_width;
-      a.v = s.v_cache + layer * s.capacity * kv_width;
-      a.kv_stride = kv_width;
-      a.rows = rows;
-      a.heads = heads;
-      a.kv_heads = kv_heads;
-      a.capacity = int(s.capacity);
-      a.device_offset = &s.control->context;
-      a.status = &s.control->status;
-      a.chunk = s.attention_chunk;
-      a.max_splits = s.attention_splits;
-      a.scratch = lead.attention_scratch + size_t(j) * scratch_floats;
-      a.out = lead.attention + size_t(j) * rows * heads * 128;
-      a.out_stride = heads * 128;
-      tick(lead);
-      tick(lead);
-      launch_verify_attention(a, lead.stream, pdl);
-    }
+    QkvParams q{};
+    q.qkv = lead.qkv;
+    q.rows = total;
+    q.heads = heads;
+    q.kv_heads = kv_heads;
+    q.qkv_stride = qkv_width;
+    q.q_norm = c.qk_norm ? L.q_norm : nullptr;
+    q.k_norm = c.qk_norm ? L.k_norm : nullptr;
+    q.eps = c.rms_norm_eps;
+    q.rope_table = m.rope_table;
+    q.max_positions = int(c.max_position_embeddings);
+    q.slots = batch.slots;
+    q.rows_per_session = rows;
+    q.layer = int(layer);
+    tick(lead);
+    launch_qk_norm_rope_store(q, lead.stream, pdl);
+    // Chunks, splits and merge of the single-session step: every session ends with the bits its own step gives.
+    AttentionParams a{};
+    a.q = lead.qkv;
+    a.q_stride = qkv_width;
+    a.kv_stride = kv_width;
+    a.rows = rows;
+    a.heads = heads;
+    a.kv_heads = kv_heads;
+    a.chunk = lead.attention_chunk;
+    a.max_splits = lead.attention_splits;
+    a.scratch = lead.attention_scratch;
+    a.scratch_stride = scratch_floats;
+    a.out = lead.attention;
+    a.out_stride = heads * 128;
+    a.slots = batch.slots;
+    a.maps = batch.maps;
+    a.status = &lead.control->status;
+    a.sessions = count;
+    a.layer = int(layer);
+    a.merge_blocks = true;
+    tick(lead);
+    tick(lead);
+    launch_verify_attention(a, lead.stream, pdl);
     run_projection_residual_norm(lead, L.o, lead.attention, total, L.ffn_norm, pdl);
     if (has_plan(lead, L.gate_up, total, kEpiSiluPair)) {
       run_linear(lead, L.gate_up, lead.normed, total, kEpiSiluPair, lead.act, ffn, pdl);
@@ -910,12 +905,9 @@ void enqueue_batch_step(ei_batch& batch, int rows) {
                            lead.stream, pdl);
   }
   // Greedy token, acceptance and commit per session, on its own rows of the per-block partials.
-  for (int j = 0; j < count; ++j) {
-    ei_session& s = *batch.sessions[j];
-    tick(lead);
-    launch_finalize(lead.best_value + j * rows, lead.best_index + j * rows, parts, rows, lead.targets + j * rows,
-                    lead.step_tokens + j * rows, s.control, nullptr, nullptr, nullptr, lead.stream, pdl);
-  }
+  tick(lead);
+  launch_finalize_wide(lead.best_value, lead.best_index, parts, 16, 1, rows, count, lead.targets, lead.step_tokens,
+                       batch.slots, lead.stream, pdl);
 }
 
 void ensure_wide_buffers(ei_batch& batch, size_t rows) {
@@ -1044,8 +1036,8 @@ void enqueue_wide_batch_step(ei_batch& batch, int rows) {
   launch_argmax_partials_wide(batch.logits, total, c.vocab_size, c.vocab_size, batch.best_value, batch.best_index,
                               kWideParts, lead.stream, pdl);
   tick(lead);
-  launch_finalize_wide(batch.best_value, batch.best_index, kWideParts, rows, count, batch.targets, ws.step_tokens,
-                       batch.slots, lead.stream, pdl);
+  launch_finalize_wide(batch.best_value, batch.best_index, kWideParts, 1, kWideParts, rows, count, batch.targets,
+                       ws.step_tokens, batch.slots, lead.stream, pdl);
   tick(lead);
   launch(gather_controls_kernel, dim3((count + 127) / 128), dim3(128), 0, lead.stream, pdl,
          (const SessionSlot*)batch.slots, count, batch.controls);

@@ -165,18 +165,21 @@ __global__ void __launch_bounds__(512) finalize_kernel(const float* best_value, 
   accept_commit(chosen, rows, step_tokens, control, context_length, pending, result, sink);
 }
 
-// Wide batch: one block per session, one warp per row of that session. Partials are laid out [row][parts].
+// Batches: one block per session, one warp per row of that session.
 __global__ void __launch_bounds__(512) finalize_wide_kernel(const float* best_value, const int* best_index, int parts,
-                                                            int rows, uint32_t* targets, const uint32_t* step_tokens,
+                                                            int part_stride, int row_stride, int rows, uint32_t* targets, const uint32_t* step_tokens,
                                                             const SessionSlot* slots) {
   __shared__ uint32_t chosen[16];
   grid_dependency_wait();
   const int session = blockIdx.x, row = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (row < rows) {
-    const size_t base = (size_t(session) * rows + row) * parts;
+    const size_t base = (size_t(session) * rows + row) * row_stride;
     float best = -INFINITY;
     int index = 0x7fffffff;
-    for (int part = lane; part < parts; part += 32) take_better(best, index, best_value[base + part], best_index[base + part]);
+    for (int part = lane; part < parts; part += 32) {
+      const size_t at = base + size_t(part) * part_stride;
+      take_better(best, index, best_value[at], best_index[at]);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float other = __shfl_xor_sync(0xffffffffu, best, o);
@@ -225,11 +228,11 @@ void launch_argmax_partials_wide(const bf16* logits, size_t rows, size_t vocab, 
          int(vocab), row_stride, best_value, best_index);
 }
 
-void launch_finalize_wide(const float* best_value, const int* best_index, int parts, int rows_per_session,
-                          int sessions, uint32_t* targets, const uint32_t* step_tokens, const SessionSlot* slots,
+void launch_finalize_wide(const float* best_value, const int* best_index, int parts, int part_stride, int row_stride,
+                          int rows_per_session, int sessions, uint32_t* targets, const uint32_t* step_tokens, const SessionSlot* slots,
                           cudaStream_t stream, bool pdl) {
   launch(finalize_wide_kernel, dim3(sessions), dim3(512), 0, stream, pdl, best_value, best_index, parts,
-         rows_per_session, targets, step_tokens, slots);
+         part_stride, row_stride, rows_per_session, targets, step_tokens, slots);
 }
 
 void launch_accept(const uint32_t* inputs, const uint32_t* targets, int rows, int32_t* context_length,
