@@ -3,14 +3,19 @@
 // Same skeleton as the int4 kernel (awq_tma.cuh) without the dequantisation: a tile is 8 output features over
 // one K slice of up to 4096 inputs, brought into shared memory by one tiled TMA copy (rank-3 map
 // [unit of 64 inputs][row][128 bytes], 128-byte swizzle, 64 KiB for a full slice) through a ring of stages on
-// mbarriers with bounded waits. Warp w owns inputs [256 w, 256 w + 256) of the slice; its activation fragments
+// mbarriers with bounded waits. A warp owns 256 inputs of the slice; its activation fragments
 // are loaded once, 64 contiguous bytes per row and load, and stay in registers (the register-prefetching
 // kernel in smallm_gemm.cuh keeps them in shared memory and reads them again for every MMA, which at more
 // than 8 rows costs a quarter of the HBM rate on the vocabulary head). The loop is 8 128-bit shared-memory
 // loads and 16 mma.sync.m16n8k16 per tile and warp; a lane's 16-byte chunk feeds two MMAs, and because the
 // activation fragments take their inputs from the same positions, any fixed assignment of a chunk's eight
-// inputs to MMA k-slots is valid. Per tile the 16 warps add their partial accumulators through shared memory
+// inputs to MMA k-slots is valid. Per phase the warps add their partial accumulators through shared memory
 // in a fixed order; K beyond 4096 is split over blocks (ksplit) that write FP32 partials.
+//
+// A slice of at most 2048 (1024) inputs needs eight (four) of the sixteen warps: two (four) tiles then go side by side
+// (kTiles), so that a phase - one barrier, one reduction, one epilogue - covers as many tiles and no warp idles. What
+// bounds the projections of a small decoder at one row is latency, not bytes: the 1024-input projections of the 0.6B
+// model are 3 to 5 tiles per block, each formerly a phase of its own with a quarter of the warps at work.
 #pragma once
 
 #include <cuda.h>
@@ -19,11 +24,12 @@
 
 namespace ei {
 
-constexpr int kDenseMaxStages = 8;
+constexpr int kDenseMaxStages = 12;
 constexpr int kDenseWarpInputs = 256;  // inputs of the slice one warp owns: four 64-input units
 
 struct DenseLaunch {
-  int stages;           // tiles in flight per block
+  int stages;           // tiles in flight per block, a multiple of the tiles per phase
+  int early;            // of them requested before the kernel waits for its predecessor
   int units_box;        // 64-input units the weight box covers (<= 64)
   uint32_t wait_limit;  // polls before a wait gives up (0: kAwqWaitLimit)
   uint32_t extra_tx;    // test hook: bytes the first copy is expected to deliver beyond what it does (0 in production)
@@ -43,11 +49,12 @@ __host__ __device__ inline DenseLayout dense_layout(const DenseLaunch& cfg) {
   return l;
 }
 
-template <bool kHigh>
+// kTiles (1, 2, 4): tiles per phase, kGemmWarps / kTiles warps each.
+template <bool kHigh, int kTiles>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     dense_tma_kernel(const __grid_constant__ CUtensorMap weights, const GemmParams p, const DenseLaunch cfg) {
   constexpr int kBlock = 136;
-  constexpr int kParts = 4;
+  constexpr int kTileWarps = kGemmWarps / kTiles;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_address(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
@@ -86,7 +93,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    issue(0);  // weights do not depend on the preceding kernel; more now would delay the activation loads below
+    // Weights do not depend on the preceding kernel. Few rows: the whole ring is requested now and streams while that
+    // kernel runs; with more the activation loads below would queue behind it.
+    for (int index = 0; index < cfg.early; ++index) issue(index);
   }
   __syncthreads();  // barriers initialised: synchronise while the block would wait for its predecessor anyway
   grid_dependency_wait();
@@ -94,10 +103,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   // A fragments of this warp's 256 inputs: cell (unit u, half h) of lane (g, c) holds inputs
   // [64 u + 32 h + 8 c, + 8) of rows g and g + 8: the four lanes of a row read 64 contiguous bytes per load.
-  const bool live = warp < parts;
+  const int mine = warp / kTileWarps, part_of_tile = warp % kTileWarps;  // tile of the phase, inputs of the slice
+  const bool live = part_of_tile < parts;
   uint4 lo[8], hi[8];
   {
-    const int k = (part_begin + (live ? warp : 0)) * kDenseWarpInputs + c * 8;
+    const int k = (part_begin + (live ? part_of_tile : 0)) * kDenseWarpInputs + c * 8;
 #pragma unroll
     for (int cell = 0; cell < 8; ++cell) {
       lo[cell] = make_uint4(0, 0, 0, 0);
@@ -109,23 +119,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
   asm volatile("" ::: "memory");  // the activation loads are issued before the rest of the ring is requested
   if (threadIdx.x == 0)
-    for (int s = 1; s < cfg.stages; ++s) issue(s);
+    for (int index = cfg.early; index < cfg.stages; ++index) issue(index);
 
-  // Reduction role of this lane: warp r owns accumulator elements e in [8r, 8r + 8); a lane is (part, element).
-  const int e = warp * 8 + (lane & 7);
-  const int part_index = lane >> 3;
+  // Reduction role of this thread: element e of the phase's output unit `unit` (a tile, or a gate and an up tile),
+  // share q of `shares` of its partials; the shares are neighbouring lanes.
+  const int units = kTiles == 1 ? 1 : pair ? kTiles / 2 : kTiles, shares = 4 / units;
+  const int unit = threadIdx.x / (128 * shares), e = (threadIdx.x / shares) & 127, q = threadIdx.x & (shares - 1);
   const int rl = e >> 2, reg = e & 3;
   const int row = (rl >> 2) + (reg >= 2 ? 8 : 0);
   const int col = (rl & 3) * 2 + (reg & 1);
   float best_value = -INFINITY;
   int best_index = 0x7fffffff;
-  float gate_sum = 0.0f;  // fused SwiGLU: the gate tile's sum waits here for the up tile
+  float gate_sum = 0.0f;  // fused SwiGLU, one tile per phase: the gate tile's sum waits here for the up tile
 
-  // Rows g of units 4 warp .. 4 warp + 3 in a staged tile [unit][row][128 B]; 16-byte chunk j of row r sits at
+  // Rows g of the warp's four units in a staged tile [unit][row][128 B]; 16-byte chunk j of row r sits at
   // chunk (j ^ r), and bits 4-6 of lane_base hold g, so chunk (4 h + c) of unit u is at
   // (lane_base + u * 1024) ^ ((4 h + c) << 4).
   const uint32_t stages_address = smem_address(stages);
-  const uint32_t lane_base = uint32_t(warp * 4096 + g * 128 + (g << 4));
+  const uint32_t lane_base = uint32_t(part_of_tile * 4096 + g * 128 + (g << 4));
   auto shared_u128 = [](uint32_t address) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(address));
@@ -134,16 +145,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   int slot = 0;
   uint32_t parity = 0;
-  // Giving up is the block's decision: a thread whose wait ran out raises the flag before the tile's block-wide
-  // barrier; every thread reads it after the barrier and acts on it at the top of the next tile.
+  // Giving up is the block's decision: a thread whose wait ran out raises the flag before the phase's block-wide
+  // barrier; every thread reads it after the barrier and acts on it at the top of the next phase.
   int gave_up = 0, tiles_done = 0;
-  for (int index = 0; index < item_count && !gave_up; ++index) {
-    const int item = item_begin + index;
-    const bool ok = mbarrier_wait(&full[slot], parity, wait_limit);
+  for (int index = 0, phase = 0; index < item_count && !gave_up; index += kTiles, phase ^= 1) {
+    const bool here = index + mine < item_count;
+    const bool ok = !here || mbarrier_wait(&full[slot + mine], parity, wait_limit);
     if (!ok) *failed = 1;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, other[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (live && ok) {
-      const uint32_t tile_address = stages_address + uint32_t(slot) * uint32_t(layout.tile_bytes) + lane_base;
+    if (live && here && ok) {
+      const uint32_t tile_address = stages_address + uint32_t(slot + mine) * uint32_t(layout.tile_bytes) + lane_base;
       uint4 w[8];
 #pragma unroll
       for (int cell = 0; cell < 8; ++cell)
@@ -160,43 +171,60 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       acc[0] += other[0]; acc[1] += other[1]; acc[2] += other[2]; acc[3] += other[3];
     }
-    if (++slot == cfg.stages) {
+    slot += kTiles;
+    if (slot == cfg.stages) {
       slot = 0;
       parity ^= 1;
     }
-    float* mine = part + (size_t(index & 1) * kGemmWarps + warp) * kBlock;
-    *reinterpret_cast<float4*>(mine + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    float* part_phase = part + size_t(phase) * kGemmWarps * kBlock;
+    *reinterpret_cast<float4*>(part_phase + warp * kBlock + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     __syncthreads();
-    // Every warp has finished reading this stage: refill it with the tile `stages` ahead.
-    if (threadIdx.x == 0) issue(index + cfg.stages);
+    // Every warp has finished reading these stages: refill them with the tiles `stages` ahead.
+    if (threadIdx.x == 0)
+      for (int t = 0; t < kTiles; ++t) issue(index + cfg.stages + t);
     gave_up = *failed;
-    tiles_done = index + 1;
+    tiles_done = index + kTiles;
 
-    // Fixed-order reduction by all 16 warps: part q adds the partials of warps q, q + 4, q + 8, q + 12 in that
-    // order and the parts are combined by two shuffles, so an output sees the same additions in every run.
-    float sum = 0.0f;
-    {
-      const float* src = part + (size_t(index & 1) * kGemmWarps + part_index) * kBlock + e;
+    // Fixed-order reduction: share q adds the partials of its tile's warps q, q + shares, ... in that order and the
+    // shares are combined by shuffles, so an output sees the same additions in every run.
+    auto total_of = [&](int tile) {
+      const float* src = part_phase + size_t(tile) * kTileWarps * kBlock + e;
+      float sum = 0.0f;
+      if (shares == 4) {
 #pragma unroll
-      for (int w = 0; w < kGemmWarps / kParts; ++w) sum += src[size_t(w) * kParts * kBlock];
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    if (part_index == 0 && row < p.M) {
+        for (int w = 0; w < kTileWarps; w += 4) sum += src[size_t(w + q) * kBlock];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      } else if (shares == 2) {
+#pragma unroll
+        for (int w = 0; w < kTileWarps; w += 2) sum += src[size_t(w + q) * kBlock];
+      } else {
+#pragma unroll
+        for (int w = 0; w < kTileWarps; ++w) sum += src[size_t(w) * kBlock];
+      }
+      if (shares >= 2) sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      return sum;
+    };
+    auto store_pair = [&](int n, float gate, float up) {  // n: feature of the up half
+      const int out_n = n - p.N / 2;
+      if (p.bias) {
+        gate += __bfloat162float(p.bias[out_n]);
+        up += __bfloat162float(p.bias[n]);
+      }
+      p.out[size_t(row) * p.out_stride + out_n] = __float2bfloat16_rn(gated_pair_value(p.glu, p.glu_limit, gate, up));
+    };
+    const int first = pair && kTiles > 1 ? unit * 2 : unit;  // first tile of this thread's unit
+    float sum = total_of(first), up_sum = 0.0f;
+    if (pair && kTiles > 1) up_sum = total_of(first + 1);
+    const int item = item_begin + index + first;
+    if (q == 0 && row < p.M && index + first < item_count) {
       const int n = tile_of(item) * 8 + col;
       if (pair) {
-        if ((item & 1) == 0) {
+        if (kTiles > 1)
+          store_pair(tile_of(item + 1) * 8 + col, sum, up_sum);
+        else if ((item & 1) == 0)
           gate_sum = sum;
-        } else {
-          float gate = gate_sum, up = sum;
-          const int out_n = n - p.N / 2;
-          if (p.bias) {
-            gate += __bfloat162float(p.bias[out_n]);
-            up += __bfloat162float(p.bias[n]);
-          }
-          p.out[size_t(row) * p.out_stride + out_n] =
-              __float2bfloat16_rn(gated_pair_value(p.glu, p.glu_limit, gate, up));
-        }
+        else
+          store_pair(n, gate_sum, sum);
       } else if (p.epilogue == kEpiPartial) {
         p.partial[(size_t(slice) * p.M + row) * p.N + n] = sum;
       } else {
@@ -220,7 +248,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (p.status) atomicOr(p.status, 4);
       // A block never leaves while a copy into its shared memory may be in flight: give every tile still in
       // the ring its chance to land (bounded again).
-      for (int back = max(0, tiles_done - 1); back < min(item_count, tiles_done - 1 + cfg.stages); ++back)
+      for (int back = max(0, tiles_done - kTiles); back < min(item_count, tiles_done + cfg.stages); ++back)
         mbarrier_wait(&full[back % cfg.stages], uint32_t((back / cfg.stages) & 1), wait_limit);
     }
     __syncthreads();
@@ -228,31 +256,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 
   if (p.epilogue == kEpiArgmax) {
-    // An element owner always sees the same output row; fold the 8 owners of each row.
+    // An element owner always sees the same output row; warp r folds the 8 owners of row r in each unit.
     __syncthreads();
     float* values = part;
-    int* indices = reinterpret_cast<int*>(part + 128);
-    if (part_index == 0) {
-      values[e] = best_value;
-      indices[e] = best_index;
+    int* indices = reinterpret_cast<int*>(part + 128 * kTiles);
+    if (q == 0) {
+      values[unit * 128 + e] = best_value;
+      indices[unit * 128 + e] = best_index;
     }
     __syncthreads();
-    if (threadIdx.x < 16) {
-      const int want = threadIdx.x;
-      float bv = -INFINITY;
-      int bi = 0x7fffffff;
-      for (int v = 0; v < 128; ++v) {
-        const int vl = v >> 2, vr = v & 3;
-        if ((vl >> 2) + (vr >= 2 ? 8 : 0) != want) continue;
-        const float value = values[v];
-        const int index = indices[v];
-        if (value > bv || (value == bv && index < bi)) {
-          bv = value;
-          bi = index;
-        }
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+    if (lane < 8 * kTiles) {
+      const int owner = (lane >> 3) * 128 + ((warp & 7) * 4 + ((lane >> 1) & 3)) * 4 + (warp >= 8 ? 2 : 0) + (lane & 1);
+      bv = values[owner];
+      bi = indices[owner];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float value = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int index = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (value > bv || (value == bv && index < bi)) {
+        bv = value;
+        bi = index;
       }
-      p.best_value[blockIdx.x * 16 + want] = bv;
-      p.best_index[blockIdx.x * 16 + want] = bi;
+    }
+    if (lane == 0) {
+      p.best_value[blockIdx.x * 16 + warp] = bv;
+      p.best_index[blockIdx.x * 16 + warp] = bi;
     }
   }
 }

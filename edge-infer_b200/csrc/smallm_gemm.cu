@@ -245,18 +245,22 @@ bool dense_tma_eligible(const GemmPlan& plan, const GemmParams& p) {
   if (p.K % kDenseWarpInputs || !aligned_16(p.w) || p.ldw % 8 || !aligned_16(p.x) || p.x_stride % 8) return false;
   const int parts_total = p.K / kDenseWarpInputs;
   if ((parts_total + plan.ksplit - 1) / plan.ksplit > kGemmWarps) return false;
-  const DenseLaunch smallest{2, std::min(64, ((parts_total + plan.ksplit - 1) / plan.ksplit) * 4)};
+  const DenseLaunch smallest{2, 1, std::min(64, ((parts_total + plan.ksplit - 1) / plan.ksplit) * 4)};
   return dense_layout(smallest).total <= plan.smem_limit;
 }
 
 void launch_dense_tma(const GemmPlan& plan, const GemmParams& p, cudaStream_t stream, bool pdl) {
   const int parts_total = p.K / kDenseWarpInputs;
   DenseLaunch cfg{};
-  cfg.units_box = std::min(64, ((parts_total + plan.ksplit - 1) / plan.ksplit) * 4);  // the largest slice
+  const int parts = (parts_total + plan.ksplit - 1) / plan.ksplit;  // of the largest slice
+  cfg.units_box = std::min(64, parts * 4);
+  const int tiles = parts <= kGemmWarps / 4 ? 4 : parts <= kGemmWarps / 2 ? 2 : 1;
   cfg.stages = kDenseMaxStages;
   cfg.wait_limit = p.wait_limit;
   cfg.extra_tx = p.fault_tx;
-  while (cfg.stages > 2 && dense_layout(cfg).total > plan.smem_limit) --cfg.stages;
+  while (cfg.stages > 2 && (cfg.stages % tiles || dense_layout(cfg).total > plan.smem_limit)) --cfg.stages;
+  // The activations every block reads after its predecessor: up to 32 KB they are not held up by a full ring's requests.
+  cfg.early = size_t(p.M) * parts * kDenseWarpInputs * 2 <= 32 * 1024 ? cfg.stages : 1;
   const size_t smem = dense_layout(cfg).total;
   CUtensorMap weights{};
   {
@@ -271,14 +275,14 @@ void launch_dense_tma(const GemmPlan& plan, const GemmParams& p, cudaStream_t st
   int device = 0;
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device != device) {
-    EI_CUDA(cudaFuncSetAttribute(dense_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    EI_CUDA(cudaFuncSetAttribute(dense_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    for (auto kernel : {dense_tma_kernel<true, 1>, dense_tma_kernel<true, 2>, dense_tma_kernel<true, 4>,
+                        dense_tma_kernel<false, 1>, dense_tma_kernel<false, 2>, dense_tma_kernel<false, 4>})
+      EI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured_device = device;
   }
-  if (plan.high)
-    launch(dense_tma_kernel<true>, dim3(plan.grid), dim3(kGemmThreads), smem, stream, pdl, weights, p, cfg);
-  else
-    launch(dense_tma_kernel<false>, dim3(plan.grid), dim3(kGemmThreads), smem, stream, pdl, weights, p, cfg);
+  auto kernel = plan.high ? (tiles == 4 ? dense_tma_kernel<true, 4> : tiles == 2 ? dense_tma_kernel<true, 2> : dense_tma_kernel<true, 1>)
+                          : (tiles == 4 ? dense_tma_kernel<false, 4> : tiles == 2 ? dense_tma_kernel<false, 2> : dense_tma_kernel<false, 1>);
+  launch(kernel, dim3(plan.grid), dim3(kGemmThreads), smem, stream, pdl, weights, p, cfg);
 }
 
 }  // namespace
