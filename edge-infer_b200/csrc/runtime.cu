@@ -52,10 +52,21 @@ __global__ void silu_pair_rows_vec_kernel(const bf16* gate_up, int rows, int ffn
     const uint4 u = *reinterpret_cast<const uint4*>(gate_up + size_t(row) * 2 * ffn + ffn + n);
     const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
     uint32_t packed[4];
+    // The branches for tiny and very negative gates are taken only where one of the eight needs them.
+    bool rare = false;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      packed[j] = pack_bf16(silu_multiply_value(bf16_lo(gw[j]), bf16_lo(uw[j])),
-                            silu_multiply_value(bf16_hi(gw[j]), bf16_hi(uw[j])));
+    for (int j = 0; j < 4; ++j) rare |= silu_is_rare(bf16_lo(gw[j])) || silu_is_rare(bf16_hi(gw[j]));
+    if (rare) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        packed[j] = pack_bf16(silu_multiply_value(bf16_lo(gw[j]), bf16_lo(uw[j])),
+                              silu_multiply_value(bf16_hi(gw[j]), bf16_hi(uw[j])));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        packed[j] = pack_bf16(silu_multiply_common(bf16_lo(gw[j]), bf16_lo(uw[j])),
+                              silu_multiply_common(bf16_hi(gw[j]), bf16_hi(uw[j])));
+    }
     *reinterpret_cast<uint4*>(out + size_t(row) * ffn + n) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
   }
 }

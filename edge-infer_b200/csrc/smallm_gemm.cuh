@@ -100,10 +100,20 @@ __device__ __forceinline__ float silu_value(float x) {
   return __fdividef(x, 1.0f + __expf(-x));
 }
 
-__device__ __forceinline__ float silu_multiply_value(float gate, float up) {
-  const float activated = round_bf16(silu_value(gate));
+// True where silu_value leaves its main branch.
+__device__ __forceinline__ bool silu_is_rare(float x) {
+  return (__float_as_uint(x) & 0x7fffffffu) <= 0x01000000u || x < -80.0f;
+}
+__device__ __forceinline__ float multiply_activated(float activated, float up) {
   const float zero = __uint_as_float((__float_as_uint(activated) ^ __float_as_uint(up)) & 0x80000000u);
   return round_bf16(__fmaf_ieee_rn(activated, up, zero));
+}
+__device__ __forceinline__ float silu_multiply_value(float gate, float up) {
+  return multiply_activated(round_bf16(silu_value(gate)), up);
+}
+// The same for a gate that is not rare.
+__device__ __forceinline__ float silu_multiply_common(float gate, float up) {
+  return multiply_activated(round_bf16(__fdividef(gate, 1.0f + __expf(-gate))), up);
 }
 
 __device__ __forceinline__ float clamped_glu_value(float gate, float up, float limit) {
