@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   }
   // Last visible token of each row (causal): offset + r.
   const int limit_lo = offset + r_lo, limit_hi = offset + r_hi;
-  const float scale = rsqrtf(float(kDim));
+  const float scale = rsqrtf(float(kDim)), exponent_scale = scale * kLog2e;
 
   float o[16][4];
 #pragma unroll
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
     unsigned char* ks = smem + size_t(stage) * kStageBytes;
     unsigned char* vs = ks + kTileBytes;
     const int first = start + tile * kTile;
+    const bool masked = first + kTile - 1 > offset;
     if (end - first < kTile) {
       // The last tile reaches past the live rows: what the copy brought for them is whatever the cache holds
       // there (rows of rejected drafts, or memory never written). Their scores are masked below; their V rows
@@ -174,49 +175,61 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
         mma_bf16_16816(s[j], qa[2 * pair + 1][0], qa[2 * pair + 1][1], qa[2 * pair + 1][2], qa[2 * pair + 1][3], b2, b3);
       }
     }
-    // Scale, mask (causal and beyond-the-end), running maximum.
-    float tile_max_lo = -INFINITY, tile_max_hi = -INFINITY;
+    // Mask (causal and beyond-the-end; only tiles that reach past the first row's position have something to hide),
+    // running maximum of the unscaled scores: the scale and the change of base go into the exponent's one FMA. (With the
+    // rescaling left out where no maximum moved: 3 drafts behind 30 000 tokens on the 8B model 2979 -> 2937 us.)
+    if (masked) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int t0 = first + j * 8 + 2 * c, t1 = t0 + 1;
+        if (t0 > limit_lo) s[j][0] = -INFINITY;
+        if (t1 > limit_lo) s[j][1] = -INFINITY;
+        if (t0 > limit_hi) s[j][2] = -INFINITY;
+        if (t1 > limit_hi) s[j][3] = -INFINITY;
+      }
+    }
+    float new_lo = m_lo, new_hi = m_hi;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int t0 = first + j * 8 + 2 * c, t1 = t0 + 1;
-      s[j][0] = t0 <= limit_lo ? s[j][0] * scale : -INFINITY;
-      s[j][1] = t1 <= limit_lo ? s[j][1] * scale : -INFINITY;
-      s[j][2] = t0 <= limit_hi ? s[j][2] * scale : -INFINITY;
-      s[j][3] = t1 <= limit_hi ? s[j][3] * scale : -INFINITY;
-      tile_max_lo = fmaxf(tile_max_lo, fmaxf(s[j][0], s[j][1]));
-      tile_max_hi = fmaxf(tile_max_hi, fmaxf(s[j][2], s[j][3]));
+      new_lo = fmaxf(new_lo, fmaxf(s[j][0], s[j][1]));
+      new_hi = fmaxf(new_hi, fmaxf(s[j][2], s[j][3]));
     }
-    tile_max_lo = fmaxf(tile_max_lo, __shfl_xor_sync(0xffffffffu, tile_max_lo, 1));
-    tile_max_lo = fmaxf(tile_max_lo, __shfl_xor_sync(0xffffffffu, tile_max_lo, 2));
-    tile_max_hi = fmaxf(tile_max_hi, __shfl_xor_sync(0xffffffffu, tile_max_hi, 1));
-    tile_max_hi = fmaxf(tile_max_hi, __shfl_xor_sync(0xffffffffu, tile_max_hi, 2));
-    const float new_lo = fmaxf(m_lo, tile_max_lo), new_hi = fmaxf(m_hi, tile_max_hi);
-    // A row with nothing visible yet keeps m = -inf; use 0 as the exponent base so exp() gives 0.
-    const float base_lo = new_lo == -INFINITY ? 0.0f : new_lo;
-    const float base_hi = new_hi == -INFINITY ? 0.0f : new_hi;
-    const float rescale_lo = __expf(m_lo - base_lo), rescale_hi = __expf(m_hi - base_hi);
-    m_lo = new_lo;
-    m_hi = new_hi;
+    new_lo = fmaxf(new_lo, __shfl_xor_sync(0xffffffffu, new_lo, 1));
+    new_lo = fmaxf(new_lo, __shfl_xor_sync(0xffffffffu, new_lo, 2));
+    new_hi = fmaxf(new_hi, __shfl_xor_sync(0xffffffffu, new_hi, 1));
+    new_hi = fmaxf(new_hi, __shfl_xor_sync(0xffffffffu, new_hi, 2));
+    // A row with nothing visible yet keeps m = -inf; use 0 as the exponent base so that the power is 0.
+    const float top_lo = new_lo == -INFINITY ? 0.0f : new_lo, top_hi = new_hi == -INFINITY ? 0.0f : new_hi;
+    const float base_lo = top_lo * exponent_scale, base_hi = top_hi * exponent_scale;
+    // A row whose maximum stays gets a factor of exactly 1, so its bits do not depend on the other rows of the warp.
+    if (__any_sync(0xffffffffu, new_lo != m_lo || new_hi != m_hi)) {
+      const float rescale_lo = power_of_two((m_lo - top_lo) * exponent_scale);
+      const float rescale_hi = power_of_two((m_hi - top_hi) * exponent_scale);
+      l_lo *= rescale_lo;
+      l_hi *= rescale_hi;
+#pragma unroll
+      for (int d = 0; d < 16; ++d) {
+        o[d][0] *= rescale_lo;
+        o[d][1] *= rescale_lo;
+        o[d][2] *= rescale_hi;
+        o[d][3] *= rescale_hi;
+      }
+      m_lo = new_lo;
+      m_hi = new_hi;
+    }
     float sum_lo = 0.0f, sum_hi = 0.0f;
     uint32_t pa[8][2];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float p0 = __expf(s[j][0] - base_lo), p1 = __expf(s[j][1] - base_lo);
-      const float p2 = __expf(s[j][2] - base_hi), p3 = __expf(s[j][3] - base_hi);
+      const float p0 = power_of_two(fmaf(s[j][0], exponent_scale, -base_lo)), p1 = power_of_two(fmaf(s[j][1], exponent_scale, -base_lo));
+      const float p2 = power_of_two(fmaf(s[j][2], exponent_scale, -base_hi)), p3 = power_of_two(fmaf(s[j][3], exponent_scale, -base_hi));
       sum_lo += p0 + p1;
       sum_hi += p2 + p3;
       pa[j][0] = pack_bf16(p0, p1);
       pa[j][1] = pack_bf16(p2, p3);
     }
-    l_lo = l_lo * rescale_lo + sum_lo;  // per-lane partial; the quad is summed at the end
-    l_hi = l_hi * rescale_hi + sum_hi;
-#pragma unroll
-    for (int d = 0; d < 16; ++d) {
-      o[d][0] *= rescale_lo;
-      o[d][1] *= rescale_lo;
-      o[d][2] *= rescale_hi;
-      o[d][3] *= rescale_hi;
-    }
+    l_lo += sum_lo;  // per-lane partial; the quad is summed at the end
+    l_hi += sum_hi;
     // O += P V : k-step t covers tokens 16t..16t+15, n-tile d covers dims 8d..8d+7.
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -274,7 +287,7 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
 #pragma unroll
     for (int d = 0; d < 16; ++d) *reinterpret_cast<float2*>(dst + d * 8 + 2 * c) = make_float2(o[d][0], o[d][1]);
     if (c == 0) {
-      dst[128] = m_lo;
+      dst[128] = m_lo * scale;
       dst[129] = l_lo;
     }
   }
@@ -283,7 +296,7 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
 #pragma unroll
     for (int d = 0; d < 16; ++d) *reinterpret_cast<float2*>(dst + d * 8 + 2 * c) = make_float2(o[d][2], o[d][3]);
     if (c == 0) {
-      dst[128] = m_hi;
+      dst[128] = m_hi * scale;
       dst[129] = l_hi;
     }
   }

@@ -125,6 +125,14 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// 2^x by the hardware's approximation (what the fast exponential is made of); results below the normal range are 0.
+constexpr float kLog2e = 1.4426950408889634f;
+__device__ __forceinline__ float power_of_two(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 #endif  // __CUDACC__
 
 // ----------------------------------------------------------------------- launch helper
