@@ -47,6 +47,11 @@ double prompt_cycles(bool awq, const PromptTile& t, int ksplit, int rows, int N,
   const long long waves = (blocks + multiprocessors - 1) / multiprocessors;
   const int k_blocks = (K / kPromptBlockK + ksplit - 1) / ksplit;
   double cycles = 2500.0 + waves * (k_blocks * block + 2500.0 + 6.0 * t.feature_tiles * tokens);
+  // Weights beyond what L2 keeps come from HBM (about 3400 bytes a cycle) once per group of tokens: the vocabulary head
+  // of the 7B shape over 320 rows takes 321 us in one group of two token tiles, 418 us in two groups.
+  const double weights = double(N) * K * (awq ? 0.5 : 2.0);
+  const int passes = weights > 64e6 ? (rows + tokens - 1) / tokens : 1;
+  cycles = std::max(cycles, passes * weights / 3400.0 + 4000.0);
   if (partial) cycles += double(ksplit) * rows * N * 8.0 / 3000.0;  // FP32 sums out and in again, through L2
   if (store && ksplit > 1) cycles += 4000.0;                        // one more kernel
   return cycles;
