@@ -15,7 +15,8 @@
 // A slice of at most 2048 (1024) inputs needs eight (four) of the sixteen warps: two (four) tiles then go side by side
 // (kTiles), so that a phase - one barrier, one reduction, one epilogue - covers as many tiles and no warp idles. What
 // bounds the projections of a small decoder at one row is latency, not bytes: the 1024-input projections of the 0.6B
-// model are 3 to 5 tiles per block, each formerly a phase of its own with a quarter of the warps at work.
+// model are 3 to 5 tiles per block, each formerly a phase of its own with a quarter of the warps at work. One token of that
+// model 843 -> 808 us, of the 1024-wide layered decoder 946 -> 886 us (with the ring requested early, below).
 #pragma once
 
 #include <cuda.h>

@@ -254,6 +254,7 @@ void launch_dense_tma(const GemmPlan& plan, const GemmParams& p, cudaStream_t st
   DenseLaunch cfg{};
   const int parts = (parts_total + plan.ksplit - 1) / plan.ksplit;  // of the largest slice
   cfg.units_box = std::min(64, parts * 4);
+  // Tiles side by side: as many as the sixteen warps hold at one warp per 256 inputs.
   const int tiles = parts <= kGemmWarps / 4 ? 4 : parts <= kGemmWarps / 2 ? 2 : 1;
   cfg.stages = kDenseMaxStages;
   cfg.wait_limit = p.wait_limit;
