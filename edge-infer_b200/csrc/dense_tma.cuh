@@ -22,39 +22,17 @@
 #include <cuda.h>
 
 #include "awq_tma.cuh"
+#include "dense_ring.hpp"
 
 namespace ei {
 
-constexpr int kDenseMaxStages = 12;
-constexpr int kDenseWarpInputs = 256;  // inputs of the slice one warp owns: four 64-input units
-
-struct DenseLaunch {
-  int stages;           // tiles in flight per block, a multiple of the tiles per phase
-  int early;            // of them requested before the kernel waits for its predecessor
-  int units_box;        // 64-input units the weight box covers (<= 64)
-  uint32_t wait_limit;  // polls before a wait gives up (0: kAwqWaitLimit)
-  uint32_t extra_tx;    // test hook: bytes the first copy is expected to deliver beyond what it does (0 in production)
-};
-
-struct DenseLayout {
-  int tile_bytes;
-  size_t stage_offset, part_offset, barrier_offset, total;
-};
-__host__ __device__ inline DenseLayout dense_layout(const DenseLaunch& cfg) {
-  DenseLayout l;
-  l.tile_bytes = cfg.units_box * 1024;
-  l.stage_offset = 0;
-  l.part_offset = size_t(cfg.stages) * l.tile_bytes;
-  l.barrier_offset = l.part_offset + size_t(2) * kGemmWarps * 136 * sizeof(float);
-  l.total = l.barrier_offset + 128 + 1024;  // + slack to reach a 1024-byte boundary
-  return l;
-}
+static_assert(kDenseWarps == kGemmWarps, "the ring is laid out for the block of these kernels");
 
 // kTiles (1, 2, 4): tiles per phase, kGemmWarps / kTiles warps each.
 template <bool kHigh, int kTiles>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     dense_tma_kernel(const __grid_constant__ CUtensorMap weights, const GemmParams p, const DenseLaunch cfg) {
-  constexpr int kBlock = 136;
+  constexpr int kBlock = kDensePartBlock;
   constexpr int kTileWarps = kGemmWarps / kTiles;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_address(smem_raw) & 1023u)) & 1023u);

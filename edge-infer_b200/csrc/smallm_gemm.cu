@@ -240,26 +240,28 @@ void launch_awq(const GemmPlan& plan, const GemmParams& p, cudaStream_t stream, 
   dispatch_awq(plan.high, pair, cfg.tma_sz != 0, full && cfg.tma_sz != 0, plan.grid, smem, stream, pdl, maps, p, cfg);
 }
 
+// Steps of 256 inputs in the largest K slice.
+int dense_slice_parts(const GemmPlan& plan, const GemmParams& p) {
+  return (p.K / kDenseWarpInputs + plan.ksplit - 1) / plan.ksplit;
+}
+
 // The TMA-fed BF16 kernel takes weights whose rows are 16-byte aligned and K in steps of a warp's 256 inputs.
 bool dense_tma_eligible(const GemmPlan& plan, const GemmParams& p) {
   if (p.K % kDenseWarpInputs || !aligned_16(p.w) || p.ldw % 8 || !aligned_16(p.x) || p.x_stride % 8) return false;
-  const int parts_total = p.K / kDenseWarpInputs;
-  if ((parts_total + plan.ksplit - 1) / plan.ksplit > kGemmWarps) return false;
-  const DenseLaunch smallest{2, 1, std::min(64, ((parts_total + plan.ksplit - 1) / plan.ksplit) * 4)};
-  return dense_layout(smallest).total <= plan.smem_limit;
+  const int parts = dense_slice_parts(plan, p);
+  return parts <= kGemmWarps && dense_ring(parts, plan.smem_limit).tiles > 0;
 }
 
 void launch_dense_tma(const GemmPlan& plan, const GemmParams& p, cudaStream_t stream, bool pdl) {
-  const int parts_total = p.K / kDenseWarpInputs;
   DenseLaunch cfg{};
-  const int parts = (parts_total + plan.ksplit - 1) / plan.ksplit;  // of the largest slice
-  cfg.units_box = std::min(64, parts * 4);
-  // Tiles side by side: as many as the sixteen warps hold at one warp per 256 inputs.
-  const int tiles = parts <= kGemmWarps / 4 ? 4 : parts <= kGemmWarps / 2 ? 2 : 1;
-  cfg.stages = kDenseMaxStages;
+  const int parts = dense_slice_parts(plan, p);
+  const DenseRing ring = dense_ring(parts, plan.smem_limit);
+  const int tiles = ring.tiles;
+  if (!tiles) throw std::invalid_argument("small-M BF16 GEMM does not fit in shared memory");
+  cfg.stages = ring.stages;
+  cfg.units_box = dense_units_box(parts);
   cfg.wait_limit = p.wait_limit;
   cfg.extra_tx = p.fault_tx;
-  while (cfg.stages > 2 && (cfg.stages % tiles || dense_layout(cfg).total > plan.smem_limit)) --cfg.stages;
   // The activations every block reads after its predecessor: up to 32 KB they are not held up by a full ring's requests.
   cfg.early = size_t(p.M) * parts * kDenseWarpInputs * 2 <= 32 * 1024 ? cfg.stages : 1;
   const size_t smem = dense_layout(cfg).total;
