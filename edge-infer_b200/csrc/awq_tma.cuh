@@ -480,8 +480,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     // the next phase, so the read costs the phase nothing).
     if (!ok) *failed = 1;
     __syncthreads();
-    // Every warp has finished reading these stages: refill them with the tiles `stages` ahead.
-    if (threadIdx.x == 0) issue(step + ring_phases);  // lands in the slot this phase has just left
+    // Every warp has finished reading these stages: refill them with the tiles `stages` ahead. Not where this thread's own
+    // wait ran out: a barrier whose phase has not completed cannot be armed again.
+    if (threadIdx.x == 0 && ok) issue(step + ring_phases);  // lands in the slot this phase has just left
 #pragma unroll
     for (int t = 0; t < (kSwap ? 1 : kAwqPhaseTiles); ++t) {
       const float* src = part + ((size_t(phase) * kAwqPhaseTiles + t) * kGemmWarps + part_index) * kBlock + e;
@@ -496,8 +497,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (threadIdx.x == 0) {
       if (p.status) atomicOr(p.status, 4);
       // A block never leaves while a copy into its shared memory may be in flight: give every phase still in
-      // the ring its chance to land (bounded again).
-      for (int back = max(0, steps_done - 1); back < steps_done - 1 + ring_phases; ++back)
+      // the ring its chance to land (bounded again): those from the phase that gave up to the one requested after it, if
+      // this thread's own wait succeeded. (If not, the parity asked for last is that of a phase long past.)
+      if (kTmaSz) mbarrier_wait(sz_full, 0, wait_limit);
+      for (int back = max(0, steps_done - 1); back < steps_done + ring_phases; ++back)
         if (back * kAwqPhaseTiles < item_count)
           mbarrier_wait(&full[back % ring_phases], uint32_t((back / ring_phases) & 1), wait_limit);
     }

@@ -158,8 +158,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     float* part_phase = part + size_t(phase) * kGemmWarps * kBlock;
     *reinterpret_cast<float4*>(part_phase + warp * kBlock + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     __syncthreads();
-    // Every warp has finished reading these stages: refill them with the tiles `stages` ahead.
-    if (threadIdx.x == 0)
+    // Every warp has finished reading these stages: refill them with the tiles `stages` ahead. Not after a wait that ran
+    // out: a barrier whose phase has not completed cannot be armed again, nor could the drain below tell its copies apart.
+    if (threadIdx.x == 0 && index + cfg.stages < item_count && !*failed)
       for (int t = 0; t < kTiles; ++t) issue(index + cfg.stages + t);
     gave_up = *failed;
     tiles_done = index + kTiles;
@@ -226,8 +227,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (threadIdx.x == 0) {
       if (p.status) atomicOr(p.status, 4);
       // A block never leaves while a copy into its shared memory may be in flight: give every tile still in
-      // the ring its chance to land (bounded again).
-      for (int back = max(0, tiles_done - kTiles); back < min(item_count, tiles_done + cfg.stages); ++back)
+      // the ring (the phase that gave up and the `stages` tiles requested from there on) its chance to land (bounded again).
+      for (int back = max(0, tiles_done - kTiles); back < min(item_count, tiles_done - kTiles + cfg.stages); ++back)
         mbarrier_wait(&full[back % cfg.stages], uint32_t((back / cfg.stages) & 1), wait_limit);
     }
     __syncthreads();

@@ -1,0 +1,33 @@
+"""Bounded waits that run out in the weight-streaming kernels after they have gone round their rings (no fault, trap or
+endless loop: the first weight copy's barrier is told to expect 16 bytes more than the copy delivers, with a short poll
+limit). 128 heads of queries, keys and values are 2048 tiles of eight features, 13 or 14 a block: more than the ring of twelve
+holds, so there is a tile left to refill the failed tile's place with."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("quant", [0, 1])
+def test_a_ring_that_gave_up_is_not_refilled(cuda, package, quant):
+    syn = package.synthetic
+    shape = package.Shape(vocab_size=512, n_layers=1, n_heads=112, n_kv_heads=8, hidden_size=256, intermediate_size=512,
+                          quant_type=quant, max_position_embeddings=256)
+    model = package.Model(shape, syn.make_model(shape, seed=3))
+    session, sibling = model.new_session(64), model.new_session(64)
+    sibling.prefill([4, 5, 6])
+    session.prefill([1, 2, 3])
+    expected = session.read_logits(1).copy()
+    first = session.verify([7, 8, 9])
+    session.truncate(3)
+    for _ in range(3):
+        session.inject_wait_timeout(2000)
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            session.verify([7, 8, 9])
+        assert session.context_size() == 0
+        session.prefill([1, 2, 3])
+        assert np.array_equal(session.read_logits(1), expected)
+        again = session.verify([7, 8, 9])
+        assert again.targets == first.targets and again.emitted == first.emitted
+        session.truncate(3)
+    assert sibling.verify([7, 8]).emitted >= 1
