@@ -40,9 +40,9 @@
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
 //
 // Every wait on an mbarrier is bounded. A role whose wait runs out raises a flag in shared memory that every
-// other wait polls, so all roles leave their loops; the copy thread then waits (bounded) for its copies in
-// flight, the MMA thread for the MMAs it issued, bit 2 of GemmParams::status is set and the tensor memory is
-// freed before the block returns.
+// other wait polls, so all roles leave their loops. When all have, one thread waits (bounded) for the MMAs issued and the
+// copies in flight (prompt_drain), sets bit 2 of GemmParams::status, and the tensor memory is freed before the block
+// returns.
 #pragma once
 
 #include "awq_tma.cuh"
@@ -80,7 +80,11 @@ struct PromptShared {
   uint64_t done;
   uint32_t tmem_base;
   volatile int abort;
+  // Where the roles stopped, for prompt_drain: K blocks that the activations' and the weights' copy thread requested, and
+  // the first K block of its team that a dequantising warp did not hand over.
+  int issued[2], left[kPromptWorkerWarps];
 };
+static_assert(sizeof(PromptShared) <= kPromptSharedExtra - 1024, "the block's state lies behind the rings");
 
 // ---- tcgen05 wrappers ----------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* shared_result, uint32_t columns) {
@@ -155,6 +159,42 @@ __device__ __forceinline__ uint32_t elect_one() {
 }
 __device__ __forceinline__ void mbarrier_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_address(bar)) : "memory");
+}
+// Takes `bytes` off what the current phase still expects, as a copy that delivers them would.
+__device__ __forceinline__ void mbarrier_complete_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_address(bar)), "r"(bytes) : "memory");
+}
+
+// After every role has left, one of them early: waits until nothing writes into the block's shared or tensor memory any
+// more. A K block's `ready` also counts arrivals that the roles which left still owe (of the other copy thread, of the
+// dequantising warps); they are made up for here, so that its phase completes on the bytes of its copies alone and every
+// wait ends when they have landed. Without that the int4 form's activations could only be waited for by letting the limit
+// run out, once per stage. The bytes that the test hook expects beyond the first copy's are taken off first.
+template <bool kAwq>
+__device__ __forceinline__ void prompt_drain(PromptShared* sh, const PromptTile& tile, uint32_t extra_tx, uint32_t limit) {
+  auto landed = [&](uint64_t* bar, int kb, int stages) {
+    for (uint32_t polls = 0; polls < limit; ++polls)
+      if (mbarrier_try_wait(bar, (kb / stages) & 1)) return;
+  };
+  landed(&sh->done, 0, 1);
+  if (extra_tx) mbarrier_complete_tx(kAwq ? &sh->raw_full[0] : &sh->ready[0], extra_tx);
+  const int stages = tile.x_stages, activations = sh->issued[0], weights = sh->issued[1];
+  if (kAwq)
+    for (int kb = max(0, weights - tile.raw_stages); kb < weights; ++kb)
+      landed(&sh->raw_full[kb % tile.raw_stages], kb, tile.raw_stages);
+  const int last = kAwq ? activations : max(activations, weights);
+  for (int kb = max(0, last - stages); kb < last; ++kb) {
+    uint64_t* const bar = &sh->ready[kb % stages];
+    int owed = 0;
+    if (kAwq) {
+      const int* const left = sh->left + kb % tile.w_stages * kPromptTeamWarps;
+      for (int w = 0; w < kPromptTeamWarps; ++w) owed += left[w] <= kb;
+    } else {
+      owed = (activations <= kb) + (weights <= kb);
+    }
+    for (; owed > 0; --owed) mbarrier_arrive(bar);
+    landed(bar, kb, stages);
+  }
 }
 
 template <bool kAwq>
@@ -246,15 +286,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
           parity ^= 1;
         }
       }
-      if (sh->abort) {
-        // Copies still in flight write into this block's shared memory: wait for them (bounded) before leaving.
-        // The weights of K block 0 carry the test hook's unmet expectation and are known never to complete.
-        for (int kb = max(p.fault_tx ? 1 : 0, issued - stages); kb < issued; ++kb) {
-          const int s = kb % stages;
-          for (uint32_t polls = 0; polls < limit; ++polls)
-            if (mbarrier_try_wait(&full[s], (kb / stages) & 1)) break;
-        }
-      }
+      sh->issued[weights ? 1 : 0] = issued;
     }
   } else if (warp > kPromptWorkerWarps) {
     // ---- MMA warps: warp i issues for the accumulators i, i + issuers, ... (feature tile major). The whole warp walks
@@ -263,7 +295,6 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
     grid_launch_dependents();
     const int mine = __shfl_sync(0xffffffffu, warp - (kPromptWorkerWarps + 1), 0);
     if (mine < issuers) {
-      bool issued = false;
       const uint32_t leader = elect_one();
       const uint32_t instruction = prompt_instruction(columns);
       const int live = feature_tiles * token_tiles, second = mine + issuers;  // at most two accumulators per warp
@@ -292,7 +323,6 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
           }
           tcgen05_commit(&sh->empty[slot]);
         }
-        issued = true;
         w_at += w_step;
         x_at += x_step;
         if (++w_slot == p.prompt.w_stages) {
@@ -305,13 +335,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
           parity ^= 1;
         }
       }
-      if (leader) {
-        tcgen05_commit(&sh->done);  // arrives when every MMA issued so far has completed
-        if (sh->abort && issued) {
-          for (uint32_t polls = 0; polls < limit; ++polls)
-            if (mbarrier_try_wait(&sh->done, 0)) break;
-        }
-      }
+      if (leader) tcgen05_commit(&sh->done);  // arrives when every MMA issued so far has completed
     }
   } else {
     // ---- workers: dequantisation (int4 only), then the epilogue ----
@@ -341,7 +365,8 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
       // `empty` is at least as long as that of the operands, so the phase waited for is the next one to complete.
       int raw_slot = team, ready_slot = team, left_slot = team;
       uint32_t raw_parity = 0, left_parity = 0;
-      for (int kb = team; kb < end; kb += teams) {
+      int kb = team;
+      for (; kb < end; kb += teams) {
         const uint32_t scale2 = scale_next * 0x10001u, zero2 = (0x4300u | ((zero_next >> zero_shift) & 15u)) * 0x10001u;
         if (kb + teams < end) request(kb + teams);
         // The loop is left by whole warps: the barriers and the votes below are warp-wide.
@@ -385,6 +410,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
           raw_parity ^= 1;
         }
       }
+      if (lane == 0) sh->left[warp] = kb;
     }
     // The dequantisation above reads weights only; the outputs below may be read by the predecessor.
     grid_dependency_wait();
@@ -434,12 +460,18 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   }
   tcgen05_fence_before();
   __syncthreads();
+  if (sh->abort) {  // no role is left to raise it: block-uniform
+    if (threadIdx.x == 0) {
+      prompt_drain<kAwq>(sh, p.prompt, p.fault_tx, limit);
+      if (p.status) atomicOr(p.status, 4);
+    }
+    __syncthreads();
+  }
   tcgen05_fence_after();
   if (warp == kPromptWorkerWarps + 1) {
     __syncwarp();
     tmem_dealloc(tmem, kPromptTmemColumns);
   }
-  if (threadIdx.x == 0 && sh->abort && p.status) atomicOr(p.status, 4);
 }
 
 }  // namespace ei

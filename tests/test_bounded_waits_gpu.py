@@ -31,3 +31,36 @@ def test_a_ring_that_gave_up_is_not_refilled(cuda, package, quant):
         assert again.targets == first.targets and again.emitted == first.emitted
         session.truncate(3)
     assert sibling.verify([7, 8]).emitted >= 1
+
+
+@pytest.mark.parametrize("quant", [0, 1])
+def test_prompt_gemm_waits_once_for_what_is_in_flight(cuda, package, quant):
+    """After a wait has run out in the prompt GEMM its copies in flight are waited for on barriers that complete with their
+    bytes: the failing call takes about one poll limit. Barriers that also need the roles that have left would let the limit
+    run out once more per stage, four to eight times. The attention kernel's failing wait, which ends after one limit, gives
+    the time of a limit."""
+    import time
+    syn = package.synthetic
+    shape = package.Shape(vocab_size=512, n_layers=1, n_heads=16, n_kv_heads=8, hidden_size=2048, intermediate_size=2048,
+                          quant_type=quant, max_position_embeddings=256)
+    model = package.Model(shape, syn.make_model(shape, seed=5))
+    session = model.new_session(256)
+    prompt = syn.make_prompt(3, 200, shape.vocab_size)
+    session.prefill(prompt)
+    expected = session.read_logits(1).copy()
+    polls = 1 << 17
+
+    def failing(arm, call):
+        session.prefill(prompt)
+        arm(polls)
+        begin = time.perf_counter()
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            call()
+        return time.perf_counter() - begin
+
+    limit = failing(session.inject_attention_wait_timeout, lambda: session.verify([7, 8, 9]))
+    taken = failing(session.inject_wait_timeout, lambda: session.prefill(prompt))
+    assert limit > 0.02
+    assert taken < 2.5 * limit, (taken, limit)
+    session.prefill(prompt)
+    assert np.array_equal(session.read_logits(1), expected)
