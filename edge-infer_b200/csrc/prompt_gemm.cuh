@@ -9,7 +9,7 @@
 // feature_tiles x 128 features (int4: 128) and token_tiles x columns tokens (columns a multiple of 16, at most 256; at
 // most 512 accumulator columns in all). So a tile is cut to the rows there are - 333 tokens are two tiles of 176, 320 are
 // one pass over the weights with two tiles of 160 - where a tile of 128 tokens as M would leave up to 127 of them empty
-// and dequantise the weights once more. The host chooses the shape from the cost of a K block (prompt_choice).
+// and dequantise the weights once more. The host chooses the shape from the cost of a K block (prompt_choice.hpp).
 // A block walks K in blocks of 64 inputs through rings of their own for activations, weights and, int4, packed weights (a
 // ring's depth has to hide its own latency only: a copy's for activations and packed weights, the way from a free operand
 // buffer through conversion and MMA for the dequantised ones):
@@ -46,26 +46,11 @@
 #pragma once
 
 #include "awq_tma.cuh"
+#include "prompt_choice.hpp"
 
 namespace ei {
 
-constexpr int kPromptFeatures = 128;   // features per feature tile = M of one MMA
-constexpr int kPromptMaxColumns = 256; // tokens per token tile = N of one MMA, at most
-constexpr int kPromptTmemColumns = 512;
-constexpr int kPromptBlockK = 64;      // inputs per stage: one 128-byte swizzle row of BF16
-constexpr int kPromptMaxStages = 8;
-constexpr int kPromptWorkerWarps = 16;
-constexpr int kPromptTeamWarps = 4;    // int4: a team of warps dequantises a K block of the one feature tile
 constexpr int kPromptThreads = (kPromptWorkerWarps + 4) * 32;
-constexpr int kPromptWeightBytes = kPromptFeatures * kPromptBlockK * 2;             // 16 KiB BF16 operand per feature tile
-constexpr int kPromptRawBytes = kPromptFeatures * (kPromptBlockK / 2);              // 4 KiB of int4 per feature tile
-constexpr size_t kPromptSharedExtra = 1024 /* alignment */ + 512;
-
-// Bytes of the rings: activations, weight operands, packed int4 weights (every stage a multiple of 1024).
-__host__ __device__ inline int prompt_ring_bytes(const PromptTile& t) {
-  return t.x_stages * t.token_tiles * t.columns * kPromptBlockK * 2 +
-         t.feature_tiles * (t.w_stages * kPromptWeightBytes + t.raw_stages * kPromptRawBytes);
-}
 
 struct PromptMaps {
   CUtensorMap x;        // bf16 [T][K], box [columns][64], 128-byte swizzle

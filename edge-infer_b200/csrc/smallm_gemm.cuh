@@ -25,6 +25,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "prompt_choice.hpp"
 
 namespace ei {
 
@@ -43,13 +44,6 @@ enum GluKind : int {
 enum Activation : int {
   kActNone = 0,
   kActReluSquared = 1   // max(sum + bias, 0)^2, on the FP32 sum
-};
-
-// Shape of a prompt GEMM block (prompt_gemm.cuh): feature tiles of 128, token tiles of `columns` (a multiple of 16).
-struct PromptTile {
-  int feature_tiles, token_tiles, columns;
-  int x_stages, w_stages;  // K blocks of activations and of BF16 weights in the rings (x_stages >= w_stages)
-  int raw_stages;          // int4: K blocks of packed weights; a multiple of w_stages
 };
 
 struct GemmParams {
