@@ -6,6 +6,8 @@ from pathlib import Path
 
 import pytest
 
+from test_prompt_tiles_gpu import BLOCKS
+
 ROOT = Path(__file__).resolve().parents[1]
 
 PROGRAM = r"""
@@ -80,3 +82,8 @@ def choice(tmp_path_factory):
 def test_every_choice_fits_the_kernel(choice):
     result = choice()
     assert result.returncode == 0, result.stdout
+
+
+@pytest.mark.parametrize("awq,rows,n,k,slices,block", BLOCKS)
+def test_blocks_that_the_gpu_tests_are_about(choice, awq, rows, n, k, slices, block):
+    assert tuple(int(v) for v in choice(awq, rows, n, k, slices).stdout.split()) == block
