@@ -14,7 +14,6 @@ constexpr int kDensePartBlock = 136;   // floats of partial sums per warp and ph
 
 struct DenseLaunch {
   int stages;           // tiles in flight per block, a multiple of the tiles per phase
-  int early;            // of them requested before the kernel waits for its predecessor
   int units_box;        // 64-input units the weight box covers (<= 64)
   uint32_t wait_limit;  // polls before a wait gives up (0: kAwqWaitLimit)
   uint32_t extra_tx;    // test hook: bytes the first copy is expected to deliver beyond what it does (0 in production)
@@ -46,7 +45,7 @@ struct DenseRing {
 constexpr DenseRing dense_ring(int parts, size_t limit) {
   for (int tiles = parts <= kDenseWarps / 4 ? 4 : parts <= kDenseWarps / 2 ? 2 : 1; tiles >= 1; tiles /= 2) {
     int stages = kDenseMaxStages / tiles * tiles;
-    while (stages >= 2 * tiles && dense_layout(DenseLaunch{stages, 0, dense_units_box(parts), 0, 0}).total > limit)
+    while (stages >= 2 * tiles && dense_layout(DenseLaunch{stages, dense_units_box(parts), 0, 0}).total > limit)
       stages -= tiles;
     if (stages >= 2 * tiles) return DenseRing{tiles, stages};
   }

@@ -72,9 +72,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    // Weights do not depend on the preceding kernel. Few rows: the whole ring is requested now and streams while that
-    // kernel runs; with more the activation loads below would queue behind it.
-    for (int index = 0; index < cfg.early; ++index) issue(index);
+    // Weights do not depend on the preceding kernel: the whole ring is requested now and streams while that kernel runs.
+    // (With one tile now and the rest behind the activation loads a step of eight layers of 4096 takes 759 us at 8 rows and
+    // 804 at 16, instead of 733 and 768; of 2048 350.5 instead of 340.1 at one row, 411.7 instead of 407.6 at 16.)
+    for (int index = 0; index < cfg.stages; ++index) issue(index);
   }
   __syncthreads();  // barriers initialised: synchronise while the block would wait for its predecessor anyway
   grid_dependency_wait();
@@ -96,9 +97,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         hi[cell] = *reinterpret_cast<const uint4*>(p.x + size_t(g + 8) * p.x_stride + k + cell * 32);
     }
   }
-  asm volatile("" ::: "memory");  // the activation loads are issued before the rest of the ring is requested
-  if (threadIdx.x == 0)
-    for (int index = cfg.early; index < cfg.stages; ++index) issue(index);
 
   // Reduction role of this thread: element e of the phase's output unit `unit` (a tile, or a gate and an up tile),
   // share q of `shares` of its partials; the shares are neighbouring lanes.
@@ -160,7 +158,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     __syncthreads();
     // Every warp has finished reading these stages: refill them with the tiles `stages` ahead. Not after a wait that ran
     // out: a barrier whose phase has not completed cannot be armed again, nor could the drain below tell its copies apart.
-    if (threadIdx.x == 0 && index + cfg.stages < item_count && !*failed)
+    // (Of one tile a phase this thread's own wait tells.)
+    if (threadIdx.x == 0 && index + cfg.stages < item_count && (kTiles == 1 ? ok : !*failed))
       for (int t = 0; t < kTiles; ++t) issue(index + cfg.stages + t);
     gave_up = *failed;
     tiles_done = index + kTiles;
@@ -227,8 +226,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (threadIdx.x == 0) {
       if (p.status) atomicOr(p.status, 4);
       // A block never leaves while a copy into its shared memory may be in flight: give every tile still in
-      // the ring (the phase that gave up and the `stages` tiles requested from there on) its chance to land (bounded again).
-      for (int back = max(0, tiles_done - kTiles); back < min(item_count, tiles_done - kTiles + cfg.stages); ++back)
+      // the ring (the phase that gave up and the `stages` tiles requested from there on, of one tile a phase also the one
+      // requested after it; if it was not, the parity asked for is that of a phase long past) its chance to land (bounded
+      // again).
+      const int requested = tiles_done - (kTiles == 1 ? 0 : kTiles) + cfg.stages;
+      for (int back = max(0, tiles_done - kTiles); back < min(item_count, requested); ++back)
         mbarrier_wait(&full[back % cfg.stages], uint32_t((back / cfg.stages) & 1), wait_limit);
     }
     __syncthreads();

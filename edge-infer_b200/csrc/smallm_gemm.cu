@@ -262,8 +262,6 @@ void launch_dense_tma(const GemmPlan& plan, const GemmParams& p, cudaStream_t st
   cfg.units_box = dense_units_box(parts);
   cfg.wait_limit = p.wait_limit;
   cfg.extra_tx = p.fault_tx;
-  // The activations every block reads after its predecessor: up to 32 KB they are not held up by a full ring's requests.
-  cfg.early = size_t(p.M) * parts * kDenseWarpInputs * 2 <= 32 * 1024 ? cfg.stages : 1;
   const size_t smem = dense_layout(cfg).total;
   CUtensorMap weights{};
   {

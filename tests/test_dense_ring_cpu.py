@@ -17,8 +17,8 @@ int main() {
   for (int parts = 1; parts <= 16; ++parts)
     for (size_t limit = 20 * 1024; limit <= 227 * 1024; limit += 256) {
       const DenseRing r = dense_ring(parts, limit);
-      const size_t single = dense_layout(DenseLaunch{2, 0, dense_units_box(parts), 0, 0}).total;
-      const size_t total = dense_layout(DenseLaunch{r.stages, 0, dense_units_box(parts), 0, 0}).total;
+      const size_t single = dense_layout(DenseLaunch{2, dense_units_box(parts), 0, 0}).total;
+      const size_t total = dense_layout(DenseLaunch{r.stages, dense_units_box(parts), 0, 0}).total;
       bool ok = (r.tiles == 0) == (single > limit);
       if (r.tiles)
         ok = ok && r.stages % r.tiles == 0 && r.stages >= 2 * r.tiles && r.stages <= kDenseMaxStages && total <= limit &&
