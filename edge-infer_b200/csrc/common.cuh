@@ -125,7 +125,8 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// 2^x by the hardware's approximation (what the fast exponential is made of); results below the normal range are 0.
+// 2^x by the PTX instruction for it, so that e^x = 2^(x log2 e) can have its factor folded into another multiplication;
+// results below the normal range are 0.
 constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ float power_of_two(float x) {
   float y;

@@ -75,11 +75,6 @@ __device__ __forceinline__ int token_place(int t) { return 2 * (t & 3) + ((t >> 
 __device__ __forceinline__ float4 quad_at(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 times(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 // The decays' logarithms are kept to base two.
-__device__ __forceinline__ float power_of_two(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float4 exp_of(float4 a) { return make_float4(power_of_two(a.x), power_of_two(a.y), power_of_two(a.z), power_of_two(a.w)); }
 __device__ __forceinline__ float4 minus(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 __device__ __forceinline__ float4 exp_between(float4 a, float4 b) { return exp_of(minus(a, b)); }

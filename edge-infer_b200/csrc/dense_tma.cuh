@@ -15,8 +15,11 @@
 // A slice of at most 2048 (1024) inputs needs eight (four) of the sixteen warps: two (four) tiles then go side by side
 // (kTiles), so that a phase - one barrier, one reduction, one epilogue - covers as many tiles and no warp idles. What
 // bounds the projections of a small decoder at one row is latency, not bytes: the 1024-input projections of the 0.6B
-// model are 3 to 5 tiles per block, each formerly a phase of its own with a quarter of the warps at work. One token of that
-// model 843 -> 808 us, of the 1024-wide layered decoder 946 -> 886 us (with the ring requested early, below).
+// model are 3 to 5 tiles per block, each formerly a phase of its own with a quarter of the warps at work. Measured, with the
+// first few tiles of the ring requested ahead: one token of that model 837 -> 799 us, of the 1024-wide layered decoder
+// 932 -> 905 us (four tiles); two tiles instead of one, a step of four layers of 1280 inputs 163 -> 153 us at one row and
+// 192 -> 180 at eight, of 2048 inputs 212 -> 200 at one row and 229 -> 216 at five. With the whole ring requested ahead and a
+// refill that asks for less: 764 and 863 us for those two tokens.
 #pragma once
 
 #include <cuda.h>

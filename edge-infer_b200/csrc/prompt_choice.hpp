@@ -124,12 +124,16 @@ class PromptShapes {
   };
 
   // Estimated SM cycles of a launch: waves x (K blocks x the slowest of a K block's resources + the fixed part), plus
-  // what a split of K costs. Per K block: the tensor pipe needs columns / 2 cycles per MMA; shared memory moves the
+  // what a split of K costs. Per K block: the tensor pipe needs columns / 2 cycles per MMA; shared memory is charged the
   // copies in, the dequantised weights in and, per MMA, 4 KB of weights and 32 bytes per column out, 128 bytes a cycle;
   // an SM receives about 75 bytes a cycle from L2; a tile of 128 x 64 int4 weights takes about 520 cycles to dequantise.
-  // Fixed: about 5000 cycles to start, fill the rings and leave, and about 6 per accumulator column. (Measured per K block,
-  // cycles at 1.9 GHz: BF16 128 x 96 380, 256 x 112 813, 128 x 240 796; int4 128 x 112 541, 128 x 320 1005-1050, 128 x 416
-  // 1226, 128 x 256 721.)
+  // Fixed: about 5000 cycles to start, fill the rings and leave, and about 6 per accumulator column. This is an empirical
+  // cost that orders shapes, not a bandwidth limit: the charge for shared memory is above most measured K blocks (cycles at
+  // 1.9 GHz, estimate in brackets: BF16 128 x 96 380 (448), 256 x 112 813 (848), 128 x 240 796 (736); int4 128 x 112 541
+  // (520), 128 x 256 721 (800), 128 x 320 1005-1050 (1056), 128 x 416 1226 (1248)), and launches with FP32 sums come out up
+  // to a quarter above their time. Over 332 sizes with every shape and split timed, the one chosen here takes 2.5 % longer
+  // than the best in the geometric mean, 27 % at most (int4 3584 x 3584 at 512 rows, 25.8 us for 20.3). Constants fitted to
+  // those times leave 1.5 %.
   void add(const PromptTile& t) {
     const int tokens = t.token_tiles * t.columns, mmas = t.feature_tiles * t.token_tiles * (kPromptBlockK / 16);
     const double operand = t.feature_tiles * double(awq_ ? kPromptRawBytes : kPromptWeightBytes);
