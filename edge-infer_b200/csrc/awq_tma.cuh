@@ -498,7 +498,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (p.status) atomicOr(p.status, 4);
       // A block never leaves while a copy into its shared memory may be in flight: give every phase still in
       // the ring its chance to land (bounded again): those from the phase that gave up to the one requested after it, if
-      // this thread's own wait succeeded. (If not, the parity asked for last is that of a phase long past.)
+      // this thread's own wait succeeded. (If not, the parity asked for last is that of a phase long past - or, where the
+      // scales' wait ran out, of one never requested, and one more limit runs out.)
       if (kTmaSz) mbarrier_wait(sz_full, 0, wait_limit);
       for (int back = max(0, steps_done - 1); back < steps_done + ring_phases; ++back)
         if (back * kAwqPhaseTiles < item_count)
