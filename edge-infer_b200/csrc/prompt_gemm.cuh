@@ -35,7 +35,7 @@
 // cycles at any number of tokens; with warp-uniform descriptors, one barrier and one commit per K block it takes 380 and
 // 540-560 at up to 160 tokens. Above that it grows with the tile (int4 721 at 256 columns, 1005-1050 at 320, 1226 at 416,
 // counted at 1.9 GHz), and launches that fill the chip run at the rate its power sustains: 320 rows of 37888 x 3584 in
-// 65-66 us, where the sustained cuBLAS rate gives 65. Measured, int4, per launch, first form (tiles of 128 tokens as M, 256
+// 65-68 us, where the sustained cuBLAS rate gives 65. Measured, int4, per launch, first form (tiles of 128 tokens as M, 256
 // features) -> this one: 37888 x 3584, 320 rows 105 -> 66 us; 24576 x 4096, 2048 rows 344-357 -> 297-331 us (over GPUs);
 // BF16: 4096 x 2048, 333 rows 15 -> 9.9 us.
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
