@@ -14,6 +14,7 @@
 // The position of the first query row is read from device memory, so a captured graph can be
 // replayed while the context grows; blocks beyond the live length return immediately.
 #include "kernels.cuh"
+#include "prompt_attention.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -42,11 +43,8 @@ __device__ __forceinline__ int tile_offset(int token, int chunk) {
   return (chunk >> 3) * (kTile * 128) + token * 128 + (((chunk & 7) ^ (token & 7)) << 4);
 }
 
-// kDirect = false: the verify step. Block (split, kv head) covers one chunk of the sequence for all <= 16 query
-// rows and writes (o, m, l) partials for the merge kernel.
-// kDirect = true: a prompt of many rows. Block (query block, kv head) covers 16 consecutive query rows over their
-// whole causal history and writes the normalised output itself; blocks with the longest histories start first.
-template <bool kDirect>
+// Block (split, kv head) covers one chunk of the sequence for all <= 16 query rows and writes (o, m, l) partials for the
+// merge kernel.
 __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_constant__ AttentionParams p) {
   extern __shared__ unsigned char attention_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(attention_smem_raw) + 1023) &
@@ -55,7 +53,7 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   // The context length was written by the previous step; the preceding kernel of this step only appends the
   // new rows [offset, offset + rows). A chunk that ends before them can start fetching at once.
   // Wide batch (split form only): grid slice z is a session with its own cache, context length, queries, scratch.
-  const SessionSlot* owner = (!kDirect && p.slots) ? p.slots + blockIdx.z : nullptr;
+  const SessionSlot* owner = p.slots ? p.slots + blockIdx.z : nullptr;
   const int capacity = owner ? owner->capacity : p.capacity;
   const int first_offset = owner ? owner->control->context : (p.device_offset ? *p.device_offset : p.host_offset);
   // The KV heads of one stretch of tokens are neighbours in the grid, so the blocks that read the same cache rows
@@ -67,14 +65,12 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
     grid_dependency_wait();
     return;
   }
-  const int first_row = kDirect ? (int(gridDim.y) - 1 - int(blockIdx.y)) * 16 : 0;
-  const int rows = kDirect ? min(16, p.rows - first_row) : p.rows;
-  const int offset = first_offset + first_row;
+  const int rows = p.rows, offset = first_offset;
   const int length = offset + rows;
-  const int split = kDirect ? 0 : blockIdx.y;
-  const int start = kDirect ? 0 : split * p.chunk;
+  const int split = blockIdx.y;
+  const int start = split * p.chunk;
   if (start >= length) return;  // other blocks of the grid wait
-  const int end = kDirect ? length : min(start + p.chunk, length);
+  const int end = min(start + p.chunk, length);
   const int group = p.heads / p.kv_heads;
   const int stacked = rows * group;  // query rows served by this block
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
@@ -119,8 +115,8 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   const int h_hi = kv_head * group + (live_hi ? i_hi % group : 0);
   uint32_t qa[8][4];
   {
-    const bf16* q_lo = q_base + size_t(first_row + r_lo) * p.q_stride + size_t(h_lo) * kDim;
-    const bf16* q_hi = q_base + size_t(first_row + r_hi) * p.q_stride + size_t(h_hi) * kDim;
+    const bf16* q_lo = q_base + size_t(r_lo) * p.q_stride + size_t(h_lo) * kDim;
+    const bf16* q_hi = q_base + size_t(r_hi) * p.q_stride + size_t(h_hi) * kDim;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
       qa[kk][0] = live_lo ? *reinterpret_cast<const uint32_t*>(q_lo + kk * 16 + 2 * c) : 0u;
@@ -265,22 +261,6 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
 
-  if (kDirect) {
-    const float inverse_lo = l_lo > 0.0f ? 1.0f / l_lo : 0.0f, inverse_hi = l_hi > 0.0f ? 1.0f / l_hi : 0.0f;
-    if (live_lo) {
-      bf16* dst = p.out + size_t(first_row + r_lo) * p.out_stride + size_t(h_lo) * kDim;
-#pragma unroll
-      for (int d = 0; d < 16; ++d)
-        *reinterpret_cast<uint32_t*>(dst + d * 8 + 2 * c) = pack_bf16(o[d][0] * inverse_lo, o[d][1] * inverse_lo);
-    }
-    if (live_hi) {
-      bf16* dst = p.out + size_t(first_row + r_hi) * p.out_stride + size_t(h_hi) * kDim;
-#pragma unroll
-      for (int d = 0; d < 16; ++d)
-        *reinterpret_cast<uint32_t*>(dst + d * 8 + 2 * c) = pack_bf16(o[d][2] * inverse_hi, o[d][3] * inverse_hi);
-    }
-    return;
-  }
   const size_t slots = size_t(p.rows) * p.heads;
   if (live_lo) {
     float* dst = scratch + (size_t(split) * slots + size_t(r_lo) * p.heads + h_lo) * kPartial;
@@ -300,6 +280,52 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
       dst[129] = l_hi;
     }
   }
+}
+
+// A prompt of many rows: prompt_attention.cuh over the session's cache.
+struct PromptRows {
+  const AttentionParams& p;
+  int offset, rows, group, kv_head;
+  float exponent_scale;
+  bool copied_queries;
+  __device__ void request_queries(unsigned char* to, int part, int first_row, uint64_t* bar) const {
+    tma_load_5d(to, &p.q_map, 0, 0, first_row, part, kv_head, bar);
+  }
+  __device__ const bf16* query(int row, int head) const {
+    return p.q + size_t(row) * p.q_stride + size_t(kv_head * group + head) * kDim;
+  }
+  __device__ void request(unsigned char* keys, unsigned char* values, int token, uint64_t* bar) const {
+    tma_load_5d(keys, &p.k_map, 0, token, 0, kv_head, 0, bar);
+    tma_load_5d(values, &p.v_map, 0, token, 0, kv_head, 0, bar);
+  }
+  template <typename Load>
+  __device__ void finish(bool live, int row, int head, float, float sum, Load load) const {
+    const float inverse = sum > 0.0f ? 1.0f / sum : 0.0f;
+    bf16* out = p.out + size_t(row) * p.out_stride + size_t(kv_head * group + head) * kDim;
+#pragma unroll 1
+    for (int d = 0; d < kDim / 16; ++d) {
+      float v[16];
+      load(d, v);
+      if (!live) continue;
+      uint32_t packed[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) packed[i] = pack_bf16(v[2 * i] * inverse, v[2 * i + 1] * inverse);
+      uint4* dst = reinterpret_cast<uint4*>(out + d * 16);
+      dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+    }
+  }
+};
+// Blocks with the longest histories start first.
+__global__ void __launch_bounds__(kPaThreads, 1) prompt_attention_kernel(const __grid_constant__ AttentionParams p, int query_tiles) {
+  const int offset = p.device_offset ? *p.device_offset : p.host_offset;
+  if (offset < 0 || offset + p.rows > p.capacity) {
+    grid_dependency_wait();
+    return;
+  }
+  const PromptRows caller{p, offset, p.rows, p.heads / p.kv_heads, int(blockIdx.x), rsqrtf(float(kDim)) * kLog2e, p.copied_queries};
+  prompt_attention_block<kDim, false>(caller, int(gridDim.y) - 1 - int(blockIdx.y), query_tiles, p.wait_limit ? p.wait_limit : kTmaWaitLimit,
+                                      p.fault_tx, p.status);
 }
 
 // One block of four warps per (row, head). The live splits (at most 64) are read in parallel: thread s
@@ -454,10 +480,9 @@ void configure_attention_kernels() {
   int device = 0;
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device == device) return;
-  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(kAttentionShared)));
-  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(kAttentionShared)));
+  EI_CUDA(cudaFuncSetAttribute(prompt_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PaLayout<kDim>::kTotal)));
   configured_device = device;
 }
 
@@ -492,7 +517,7 @@ void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool
   configure_attention_kernels();
   const AttentionParams q = with_maps(p);
   const unsigned sessions = q.slots ? unsigned(q.sessions) : 1u;
-  launch(verify_attention_kernel<false>, dim3(q.kv_heads, q.max_splits, sessions), dim3(warps * 32), kAttentionShared,
+  launch(verify_attention_kernel, dim3(q.kv_heads, q.max_splits, sessions), dim3(warps * 32), kAttentionShared,
          stream, pdl, q);
   if (q.slots && !q.merge_blocks)
     launch(attention_merge_wide_kernel, dim3((q.rows * q.heads * q.sessions + 3) / 4), dim3(128), 0, stream, pdl, q);
@@ -501,11 +526,15 @@ void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool
 }
 
 void launch_prompt_attention(const AttentionParams& p, cudaStream_t stream, bool pdl) {
-  const int group = p.heads / p.kv_heads;
+  if (p.heads / p.kv_heads > 7)  // wider groups do not fit the step's kernel: refused here, before the first token is decoded
+    throw std::runtime_error("attention takes at most 7 query heads per key head");
   configure_attention_kernels();
-  const AttentionParams q = with_maps(p);
-  launch(verify_attention_kernel<true>, dim3(q.kv_heads, (q.rows + 15) / 16), dim3(group * 32), kAttentionShared,
-         stream, pdl, q);
+  AttentionParams q = with_maps(p);
+  q.copied_queries = encode_query_map(&q.q_map, q.q, q.rows, q.q_stride, q.heads / q.kv_heads, q.kv_heads, kDim);
+  const int stacked = q.rows * (q.heads / q.kv_heads);
+  const int query_tiles = pa_query_tiles(q.kv_heads, stacked, device_multiprocessors()), span = query_tiles * kPaRows;
+  launch(prompt_attention_kernel, dim3(q.kv_heads, (stacked + span - 1) / span), dim3(kPaThreads), PaLayout<kDim>::kTotal, stream,
+         pdl, q, query_tiles);
 }
 
 }  // namespace ei

@@ -157,6 +157,8 @@ struct AttentionParams {
   // kv_stride, kv_heads and capacity; a wide batch passes one pair per session in device memory, built with
   // encode_kv_map over all layers of the session's cache (`layer` selects the slice).
   CUtensorMap k_map, v_map;
+  CUtensorMap q_map;        // prompts: filled by the launch function if `copied_queries`
+  bool copied_queries;
   const CUtensorMap* maps;  // [sessions][2] = (K, V)
   int* status;              // optional device word; bit 2 is set if a bounded wait on a copy gave up
   uint32_t wait_limit;      // polls before a bounded wait gives up (0: the default)

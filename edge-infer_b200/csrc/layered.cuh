@@ -146,6 +146,8 @@ struct SizedAttentionParams {
   void* out;                // row r, head h at out + r * out_stride + h * vdim_pad
   int out_stride;
   CUtensorMap k_map, v_map, shared_map;  // filled by the launch functions
+  CUtensorMap q_map;        // prompt form, if `copied_queries`
+  bool copied_queries;
   int k_shift, v_shift;     // log2 of the 16-byte pieces in one row of a staged box
   int* status;
   uint32_t wait_limit, fault_tx;

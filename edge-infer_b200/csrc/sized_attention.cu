@@ -15,6 +15,7 @@
 //  * a key may end in a part that all heads share (latent attention's rotated key), fetched from a tensor of its own;
 //  * the finished output may pass a sigmoid gate.
 #include "layered_device.cuh"
+#include "prompt_attention.cuh"
 
 #include <algorithm>
 #include <stdexcept>
@@ -294,6 +295,64 @@ __global__ void __launch_bounds__(kMaxWarps * 32) sized_attention_kernel(const _
   }
 }
 
+// A prompt on prompt_attention.cuh, for keys of kKeys values and values of 128.
+template <int kKeys>
+struct SizedPromptRows {
+  const SizedAttentionParams& p;
+  int offset, rows, group, kv_head;
+  float exponent_scale;
+  bool copied_queries;
+  __device__ void request_queries(unsigned char* to, int part, int first_row, uint64_t* bar) const {
+    tma_load_5d(to, &p.q_map, 0, 0, first_row, part, kv_head, bar);
+  }
+  __device__ const bf16* query(int row, int head) const {
+    return static_cast<const bf16*>(p.q) + size_t(row) * p.q_stride + size_t(kv_head * group + head) * kKeys;
+  }
+  __device__ void request(unsigned char* keys, unsigned char* values, int token, uint64_t* bar) const {
+    tma_load_4d(keys, &p.k_map, 0, token, 0, kv_head, bar);
+    if (p.shared_pad) tma_load_4d(keys + kTile * (kKeys - p.shared_pad) * 2, &p.shared_map, 0, token, 0, 0, bar);
+    tma_load_4d(values, &p.v_map, 0, token, 0, kv_head, bar);
+  }
+  template <typename Load>
+  __device__ void finish(bool live, int row, int head, float maximum, float sum, Load load) const {
+    const int h = kv_head * group + head;
+    float f = sum > 0.0f ? p.out_scale / sum : 0.0f;
+    if (p.sink) {
+      const float m = maximum * p.scale, sink = p.sink[h], top = fmaxf(m, sink), own = __expf(m - top);
+      f = p.out_scale * own / (sum * own + __expf(sink - top));
+    }
+    bf16* out = static_cast<bf16*>(p.out) + size_t(row) * p.out_stride + size_t(h) * 128;
+    const bf16* gate = p.gate ? static_cast<const bf16*>(p.gate) + size_t(row) * p.gate_stride + size_t(h) * 128 : nullptr;
+#pragma unroll 1
+    for (int d = 0; d < 8; ++d) {
+      float v[16];
+      load(d, v);
+      if (!live) continue;
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) {
+        float a = v[i] * f, b = v[i + 1] * f;
+        if (gate) {
+          const float2 z = load_pair(gate + d * 16 + i);
+          a *= quick_sigmoid(z.x);
+          b *= quick_sigmoid(z.y);
+        }
+        store_pair(out + d * 16 + i, a, b);
+      }
+    }
+  }
+};
+template <int kKeys>
+__global__ void __launch_bounds__(kPaThreads, 1) sized_prompt_kernel(const __grid_constant__ SizedAttentionParams p, int query_tiles) {
+  const int offset = *p.device_offset;
+  if (offset < 0 || offset + p.rows > p.capacity) {
+    grid_dependency_wait();
+    return;
+  }
+  const SizedPromptRows<kKeys> caller{p, offset, p.rows, p.heads / p.kv_heads, int(blockIdx.x), p.scale * kLog2e, p.copied_queries};
+  prompt_attention_block<kKeys, true>(caller, int(gridDim.y) - 1 - int(blockIdx.y), query_tiles, p.wait_limit ? p.wait_limit : kTmaWaitLimit,
+                                      p.fault_tx, p.status);
+}
+
 // Any head size, FP32 arithmetic: one block per (row, head), a lane scores one key of a warp's 32 and the warp's lanes
 // share the value columns, kColumns each; the four warps' running sums meet in shared memory.
 template <typename T, int kColumns>
@@ -381,6 +440,29 @@ void encode_head_map(CUtensorMap* map, const void* base, int tokens, int token_s
              "sized K / V cache");
 }
 
+// The tcgen05 form: keys in whole 128-byte pieces, rows whose 16-byte pieces can be loaded at once, and a scale that
+// keeps the order of the scores.
+template <int kKeys>
+bool launch_tcgen05(const SizedAttentionParams& given, cudaStream_t stream, bool pdl) {
+  SizedAttentionParams p = given;
+  if (p.dim_pad != kKeys || p.vdim_pad != 128 || p.k_shift != 3 || p.v_shift != 3 || p.q_stride % 8 ||
+      (reinterpret_cast<uintptr_t>(p.q) & 15) || !(p.scale > 0.0f))
+    return false;
+  static thread_local int configured_device = -1;
+  int device = 0;
+  EI_CUDA(cudaGetDevice(&device));
+  if (configured_device != device) {
+    EI_CUDA(cudaFuncSetAttribute(sized_prompt_kernel<kKeys>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PaLayout<kKeys>::kTotal)));
+    configured_device = device;
+  }
+  p.copied_queries = encode_query_map(&p.q_map, p.q, p.rows, p.q_stride, p.heads / p.kv_heads, p.kv_heads, kKeys);
+  const int stacked = p.rows * (p.heads / p.kv_heads);
+  const int query_tiles = pa_query_tiles(p.kv_heads, stacked, device_multiprocessors()), span = query_tiles * kPaRows;
+  launch(sized_prompt_kernel<kKeys>, dim3(p.kv_heads, unsigned((stacked + span - 1) / span)), dim3(kPaThreads),
+         PaLayout<kKeys>::kTotal, stream, pdl, p, query_tiles);
+  return true;
+}
+
 template <int kKeys, int kValues, bool kExact>
 void launch_bucket(const SizedAttentionParams& p, bool direct, cudaStream_t stream, bool pdl) {
   static thread_local int configured_device = -1;
@@ -416,6 +498,7 @@ void launch_sized(const SizedAttentionParams& given, bool direct, cudaStream_t s
   encode_head_map(&p.k_map, p.k, tokens, p.k_stride, p.kv_heads, own, p.k_shift);
   if (p.shared_pad) encode_head_map(&p.shared_map, p.shared, tokens, p.shared_stride, 1, p.shared_pad, p.k_shift);
   encode_head_map(&p.v_map, p.v, tokens, p.v_stride, p.kv_heads, p.vdim_pad, p.v_shift);
+  if (direct && (launch_tcgen05<128>(p, stream, pdl) || launch_tcgen05<192>(p, stream, pdl))) return;
   const int widest = std::max(p.dim_pad, p.vdim_pad);
   const bool same = p.dim_pad == p.vdim_pad && p.k_shift == 3;
   if (widest <= 64) {
