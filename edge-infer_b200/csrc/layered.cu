@@ -1297,7 +1297,6 @@ void ensure_layered_workspace(ei_model& model) {
   take(ws.normed, rows * m.normed_stride * 2);
   take(ws.qkv, rows * m.max_fused * 2);
   take(ws.attention, rows * m.max_mixed * 2);
-  take(ws.gate_up, rows * m.max_gate_up * 2);
   take(ws.act, rows * m.max_ff * 2);
   take(ws.tokens, rows * 4);
   take(ws.step_tokens, rows * 4);
@@ -1473,7 +1472,7 @@ void enqueue_layered_segment(ei_session& s, int rows, size_t context) {
   auto& ws = model.prompt;
   const bool pdl = true;
   const Buffers b{rows,         ws.step_tokens, m.residual, m.linear_out,    ws.normed, ws.qkv,
-                  ws.attention, ws.gate_up,     ws.act,     m.second_normed, m.second};
+                  ws.attention, nullptr,        ws.act,     m.second_normed, m.second};
   EmbedParams token{};
   token.tokens = ws.tokens;
   token.control = s.control;
@@ -1497,9 +1496,7 @@ void enqueue_layered_segment(ei_session& s, int rows, size_t context) {
         run_prompt_linear(s, l.up, m.parallel ? m.second_normed : ws.normed, rows, ws.act, pdl);
         return;
       }
-      run_prompt_linear(s, l.gate_up, m.parallel ? m.second_normed : ws.normed, rows, ws.gate_up, pdl);
-      tick(s);
-      launch_clamped_glu<bf16>(ws.gate_up, rows, l.ff_pad, l.gate_up.glu_limit, ws.act, model.multiprocessors, s.stream, pdl);
+      run_prompt_gated(s, l.gate_up, m.parallel ? m.second_normed : ws.normed, rows, ws.act, pdl);
     };
     if (m.parallel) {
       const int mixed_ksplit = sums(l.out, ws.attention, m.mixed_partial);

@@ -67,9 +67,10 @@ class PromptShapes {
  public:
   // int4 takes one feature tile: two of them dequantise the weights of 256 features per K block, which at 128-240 columns
   // took 1500-1900 cycles where one tile with as many accumulator columns takes 1226.
-  PromptShapes(bool awq, int rows, int N, int K, int multiprocessors)
+  // `gated`: a block computes gate and up features side by side; BF16 takes a feature tile of each, int4 half a tile of each.
+  PromptShapes(bool awq, int rows, int N, int K, int multiprocessors, bool gated = false)
       : awq_(awq), rows_(rows), n_(N), k_(K), multiprocessors_(multiprocessors) {
-    for (int feature_tiles = 1; feature_tiles <= (awq ? 1 : 2); ++feature_tiles)
+    for (int feature_tiles = gated && !awq ? 2 : 1; feature_tiles <= (awq ? 1 : 2); ++feature_tiles)
       for (int token_tiles = 1; token_tiles <= 2; ++token_tiles) {
         const int most = std::min(kPromptMaxColumns, kPromptTmemColumns / (feature_tiles * token_tiles) / 16 * 16);
         const int fewest = (rows + most * token_tiles - 1) / (most * token_tiles);

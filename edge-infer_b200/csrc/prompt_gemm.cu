@@ -28,21 +28,26 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device != device) {
     EI_CUDA(cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(kPromptSharedLimit)));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kPromptSharedLimit)));
+    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kPromptSharedLimit)));
+    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(kPromptSharedLimit)));
     configured_device = device;
   }
   const int ksplit = p.epilogue == kEpiPartial ? std::max(1, p.ksplit) : 1;
-  if (p.epilogue != kEpiStore && p.epilogue != kEpiPartial)
-    throw std::invalid_argument("prompt GEMM stores BF16 outputs or FP32 partial sums");
+  const bool gated = p.epilogue == kEpiSiluPair;
+  if (p.epilogue != kEpiStore && p.epilogue != kEpiPartial && !gated)
+    throw std::invalid_argument("prompt GEMM stores BF16 outputs, gated units or FP32 partial sums");
   if (ksplit > 1 && (p.K % 128 || ksplit > p.K / 128)) throw std::invalid_argument("prompt GEMM: K split too fine");
   if (p.epilogue == kEpiPartial && (!p.partial || (reinterpret_cast<uintptr_t>(p.partial) & 15) || p.N % 4))
     throw std::invalid_argument("prompt GEMM: partial sums need a 16-byte aligned buffer");
   GemmParams q = p;
   q.ksplit = ksplit;
-  q.prompt = PromptShapes(awq, p.M, p.N, p.K, multiprocessors).best(ksplit, p.epilogue == kEpiPartial, false).tile;
+  q.prompt = PromptShapes(awq, p.M, p.N, p.K, multiprocessors, gated).best(ksplit, p.epilogue == kEpiPartial, false).tile;
   PromptMaps maps{};
   {
     const cuuint64_t dims[2] = {cuuint64_t(p.K), cuuint64_t(p.M)};
@@ -55,7 +60,7 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
     if (!aligned_16(p.qweight) || (p.K / 8) % 4) throw std::invalid_argument("prompt GEMM: packed weight rows must be 16-byte aligned");
     const cuuint64_t dims[2] = {cuuint64_t(p.K / 8), cuuint64_t(p.N)};
     const cuuint64_t strides[1] = {cuuint64_t(p.K / 8) * 4};
-    const cuuint32_t box[2] = {kPromptBlockK / 8, kPromptFeatures};
+    const cuuint32_t box[2] = {kPromptBlockK / 8, cuuint32_t(gated ? kPromptFeatures / 2 : kPromptFeatures)};
     encode_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, p.qweight, dims, strides, box,
                CU_TENSOR_MAP_SWIZZLE_NONE, "prompt int4 weights");
   } else {
@@ -69,10 +74,9 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   const int tokens = q.prompt.token_tiles * q.prompt.columns, features = kPromptFeatures * q.prompt.feature_tiles;
   const size_t shared = size_t(prompt_ring_bytes(q.prompt)) + kPromptSharedExtra;
   const dim3 grid((p.N + features - 1) / features, (p.M + tokens - 1) / tokens, ksplit);
-  if (awq)
-    launch(prompt_gemm_kernel<true>, grid, dim3(kPromptThreads), shared, stream, pdl, maps, q);
-  else
-    launch(prompt_gemm_kernel<false>, grid, dim3(kPromptThreads), shared, stream, pdl, maps, q);
+  const auto kernel = awq ? (gated ? prompt_gemm_kernel<true, true> : prompt_gemm_kernel<true, false>)
+                          : (gated ? prompt_gemm_kernel<false, true> : prompt_gemm_kernel<false, false>);
+  launch(kernel, grid, dim3(kPromptThreads), shared, stream, pdl, maps, q);
 }
 
 }  // namespace ei

@@ -38,6 +38,10 @@
 // 65-68 us, where the sustained cuBLAS rate gives 65. Measured, int4, per launch, first form (tiles of 128 tokens as M, 256
 // features) -> this one: 37888 x 3584, 320 rows 105 -> 66 us; 24576 x 4096, 2048 rows 344-357 -> 297-331 us (over GPUs);
 // BF16: 4096 x 2048, 333 rows 15 -> 9.9 us.
+// kGated: the gate and up projection of a feed-forward, whose gated units are all that leaves. Their own kernel cost a launch
+// and the pairs' way out and back (6 us at 333 x 12288, 25-37 us at 2048 x 24576); in the epilogue, which nothing overlaps, the
+// units take 23 us of the latter's 305. Whole prompts, separate -> here: 1.7B, 333 rows 2.31 -> 2.18 ms; 8B int4, 2048 rows
+// 30.8 -> 30.5; 1500 rows of the 2048-wide join decoder 8.02 -> 7.67; a batch of 64 x 5 rows, 7B int4 9.80 -> 9.57.
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
 //
 // Every wait on an mbarrier is bounded. A role whose wait runs out raises a flag in shared memory that every
@@ -116,6 +120,17 @@ __device__ __forceinline__ void tmem_load16(uint32_t address, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_load8(uint32_t address, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(address)
+               : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled operand: rows 128 bytes apart, groups of eight
 // rows 1024 bytes apart; bits [46,48) carry the descriptor version of this architecture, bits [61,64) the swizzle.
 __device__ __forceinline__ uint32_t umma_desc_low(uint32_t shared_address) {
@@ -183,7 +198,45 @@ __device__ __forceinline__ void prompt_drain(PromptShared* sh, const PromptTile&
   }
 }
 
-template <bool kAwq>
+// The gated units of kWords pairs of gate and up values, which replace the gates. Values travel as BF16 pairs, which take half
+// the conversions of single ones: the epilogue of 128 x 416 sums is bound by its instructions (two of which per unit are
+// those of the exponential and the reciprocal). The SiLU's branches for tiny and very negative gates are taken only where one
+// of the values needs them; elsewhere 1 + e^-x is far from where the fast quotient would have to scale.
+template <int kWords>
+__device__ __forceinline__ void gated_units(int glu, float limit, uint32_t (&gate)[kWords], const uint32_t (&up)[kWords]) {
+  float least = INFINITY, lowest = INFINITY;
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) {
+    least = fminf(least, fminf(fabsf(bf16_lo(gate[i])), fabsf(bf16_hi(gate[i]))));
+    lowest = fminf(lowest, fminf(bf16_lo(gate[i]), bf16_hi(gate[i])));
+  }
+  if (glu == kGluClamped) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i)
+      gate[i] = pack_bf16(clamped_glu_value(bf16_lo(gate[i]), bf16_lo(up[i]), limit),
+                          clamped_glu_value(bf16_hi(gate[i]), bf16_hi(up[i]), limit));
+  } else if (silu_is_rare(least) || silu_is_rare(lowest)) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i)
+      gate[i] = pack_bf16(silu_multiply_value(bf16_lo(gate[i]), bf16_lo(up[i])),
+                          silu_multiply_value(bf16_hi(gate[i]), bf16_hi(up[i])));
+  } else {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      auto silu = [](float x) {
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-x)));
+        return x * r;
+      };
+      const uint32_t a = pack_bf16(silu(bf16_lo(gate[i])), silu(bf16_hi(gate[i])));
+      const uint32_t signs = a ^ up[i];  // a zero of the product's sign, as in multiply_activated
+      gate[i] = pack_bf16(__fmaf_ieee_rn(bf16_lo(a), bf16_lo(up[i]), __uint_as_float((signs << 16) & 0x80000000u)),
+                          __fmaf_ieee_rn(bf16_hi(a), bf16_hi(up[i]), __uint_as_float(signs & 0x80000000u)));
+    }
+  }
+}
+
+template <bool kAwq, bool kGated>
 __global__ void __launch_bounds__(kPromptThreads, 1)
     prompt_gemm_kernel(const __grid_constant__ PromptMaps maps, const GemmParams p) {
   extern __shared__ unsigned char prompt_smem_raw[];
@@ -192,8 +245,12 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   const int columns = p.prompt.columns, block_tokens = p.prompt.token_tiles * columns;
   PromptShared* sh = reinterpret_cast<PromptShared*>(smem + prompt_ring_bytes(p.prompt));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * kPromptFeatures * p.prompt.feature_tiles, t0 = blockIdx.y * block_tokens;
-  const int feature_tiles = min(p.prompt.feature_tiles, (p.N - n0 + kPromptFeatures - 1) / kPromptFeatures);
+  // kGated: the block's rows are n0 ... of the gate and, from `pairs` on, as many of the up projection; the epilogue leaves
+  // their gated units. BF16: tile 0 is gate, tile 1 up; int4: the one tile's first and second half are.
+  const int pairs = p.N / 2;
+  const int n0 = blockIdx.x * (kPromptFeatures * p.prompt.feature_tiles / (kGated ? 2 : 1)), t0 = blockIdx.y * block_tokens;
+  const int feature_tiles =
+      kGated ? p.prompt.feature_tiles : min(p.prompt.feature_tiles, (p.N - n0 + kPromptFeatures - 1) / kPromptFeatures);
   const int token_tiles = min(p.prompt.token_tiles, (p.M - t0 + columns - 1) / columns);
   // K slice of this block (blockIdx.z of p.ksplit): whole quantisation groups, i.e. pairs of K blocks.
   const int slice = blockIdx.z;
@@ -239,12 +296,15 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
         mbarrier_expect_tx(&full[s], uint32_t(feature_tiles) * (kAwq ? kPromptRawBytes : kPromptWeightBytes) +
                                          (kb == 0 ? p.fault_tx : 0u));
         for (int f = 0; f < feature_tiles; ++f) {
-          if (kAwq)
-            tma_load_2d(raw_ring + s * raw_bytes + f * kPromptRawBytes, &maps.weights, (kb_begin + kb) * (kPromptBlockK / 8),
-                        n0 + f * kPromptFeatures, &full[s]);
-          else
+          if (kAwq) {
+            unsigned char* const to = raw_ring + s * raw_bytes + f * kPromptRawBytes;
+            const int word = (kb_begin + kb) * (kPromptBlockK / 8);
+            tma_load_2d(to, &maps.weights, word, n0 + f * kPromptFeatures, &full[s]);
+            if (kGated) tma_load_2d(to + kPromptRawBytes / 2, &maps.weights, word, pairs + n0, &full[s]);
+          } else {
             tma_load_2d(w_ring + s * w_bytes + f * kPromptWeightBytes, &maps.weights, (kb_begin + kb) * kPromptBlockK,
-                        n0 + f * kPromptFeatures, &full[s]);
+                        n0 + (kGated ? f * pairs : f * kPromptFeatures), &full[s]);
+          }
         }
       } else {
         mbarrier_expect_tx(&full[s], uint32_t(token_tiles * tile_bytes));
@@ -330,7 +390,8 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
       // w_stages, ...: every buffer belongs to one team, so no team can miss a phase of its barriers. A thread owns one
       // row: 64 inputs = 32 raw bytes = eight 16-byte chunks of the operand row.
       const int teams = p.prompt.w_stages, team = warp / kPromptTeamWarps, row = threadIdx.x & (kPromptFeatures - 1);
-      const int live_row = min(n0 + row, p.N - 1);
+      const int first_up = kPromptFeatures / 2;
+      const int live_row = min(kGated && row >= first_up ? pairs + n0 + row - first_up : n0 + row, p.N - 1);
       const bf16* scales = p.scales + size_t(live_row) * p.padded_groups;
       const int32_t* zeros = p.zeros + size_t(live_row) * p.zero_stride;
       // Scales and zero points are requested one of the team's K blocks before they are used.
@@ -407,20 +468,88 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
     const int quarter = warp & 3;
     const int tokens = min(token_tiles * columns, p.M - t0);  // live ones of this block
     constexpr int kEpilogueStep = kPromptWorkerWarps / 4 * 16;
-    if (complete) {
-      const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
-      const bool odd = lane & 1;
-      // Two neighbouring lanes (features) exchange one of two tokens' values, so that each stores a pair of features.
-      auto store_pairs = [&](const float (&v)[16], int token, int first_feature) {
+    const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
+    const bool odd = lane & 1;
+    // Two neighbouring lanes (features) exchange one of two tokens' values, so that each stores a pair of features.
+    auto store_pairs = [&](const float (&v)[16], int token, int first_feature) {
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-          const uint32_t packed = odd ? pack_bf16(other, v[i + 1]) : pack_bf16(v[i], other);
-          const int mine = token + i + (odd ? 1 : 0);
-          if (mine < p.M && first_feature < p.N)
-            *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_feature) = packed;
+      for (int i = 0; i < 16; i += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+        const uint32_t packed = odd ? pack_bf16(other, v[i + 1]) : pack_bf16(v[i], other);
+        const int mine = token + i + (odd ? 1 : 0);
+        if (mine < p.M && first_feature < p.N)
+          *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_feature) = packed;
+      }
+    };
+    // The same for pairs of two tokens' values.
+    const uint32_t halves = odd ? 0x3276u : 0x5410u;
+    auto store_words = [&](const auto& words, int token, int first_unit) {
+#pragma unroll
+      for (int i = 0; i < int(sizeof(words) / sizeof(uint32_t)); ++i) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, words[i], 1);
+        const int mine = token + 2 * i + (odd ? 1 : 0);
+        if (mine < p.M && first_unit < pairs)
+          *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_unit) = __byte_perm(words[i], other, halves);
+      }
+    };
+    if (kGated && !kAwq && complete) {
+      // A lane has a unit's gate in one accumulator and its up value in the other.
+      const int unit = n0 + quarter * 32 + lane;
+      const float gate_bias = p.bias && unit < pairs ? __bfloat162float(p.bias[unit]) : 0.0f;
+      const float up_bias = p.bias && unit < pairs ? __bfloat162float(p.bias[pairs + unit]) : 0.0f;
+#pragma unroll 1
+      for (int c = (warp >> 2) * 16; c < tokens; c += kEpilogueStep) {
+        float gate[16], up[16];
+        tmem_load16(lane_base + c, gate);
+        tmem_load16(lane_base + block_tokens + c, up);
+        uint32_t gates[8], ups[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          gates[i] = pack_bf16(gate[2 * i] + gate_bias, gate[2 * i + 1] + gate_bias);
+          ups[i] = pack_bf16(up[2 * i] + up_bias, up[2 * i + 1] + up_bias);
         }
-      };
+        gated_units(p.glu, p.glu_limit, gates, ups);
+        store_words(gates, t0 + c, unit & ~1);
+      }
+    } else if (kGated && kAwq) {
+      // A unit's gate is in lane l of the first two quarters, its up value in the same lane two quarters on: the two warps
+      // hand one another half the tokens of each group of 16 through the rings, which nothing uses any more, and each
+      // finishes the other half.
+      const bool has_up = quarter >= 2;
+      const int unit = n0 + (quarter & 1) * 32 + lane;
+      const float bias = p.bias && unit < pairs ? __bfloat162float(p.bias[has_up ? pairs + unit : unit]) : 0.0f;
+      uint4* const sent = reinterpret_cast<uint4*>(smem) + warp * 32 + lane;
+      const uint4* const received = reinterpret_cast<const uint4*>(smem) + (warp ^ 2) * 32 + lane;
+      const int mine = has_up ? 8 : 0;
+      if (complete) {
+#pragma unroll 1
+        for (int c = (warp >> 2) * 16, at = 0; c < tokens; c += kEpilogueStep, at += kPromptWorkerWarps * 32) {
+          float v[8];
+          tmem_load8(lane_base + c + (8 - mine), v);
+          sent[at] = make_uint4(pack_bf16(v[0] + bias, v[1] + bias), pack_bf16(v[2] + bias, v[3] + bias),
+                                pack_bf16(v[4] + bias, v[5] + bias), pack_bf16(v[6] + bias, v[7] + bias));
+        }
+      }
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 2) * 2 + (warp & 1)) : "memory");
+      if (complete) {
+#pragma unroll 1
+        for (int c = (warp >> 2) * 16, at = 0; c < tokens; c += kEpilogueStep, at += kPromptWorkerWarps * 32) {
+          float v[8];
+          tmem_load8(lane_base + c + mine, v);
+          const uint4 others = received[at];
+          const uint32_t words[4] = {others.x, others.y, others.z, others.w};
+          uint32_t gates[4], ups[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t own = pack_bf16(v[2 * i] + bias, v[2 * i + 1] + bias);
+            gates[i] = has_up ? words[i] : own;
+            ups[i] = has_up ? own : words[i];
+          }
+          gated_units(p.glu, p.glu_limit, gates, ups);
+          store_words(gates, t0 + c + mine, unit & ~1);
+        }
+      }
+    } else if (!kGated && complete) {
       for (int f = 0; f < feature_tiles; ++f) {
         const int feature = n0 + f * kPromptFeatures + quarter * 32 + lane;
         const float bias = p.bias && feature < p.N ? __bfloat162float(p.bias[feature]) : 0.0f;

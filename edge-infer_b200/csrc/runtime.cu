@@ -41,36 +41,6 @@ __global__ void silu_pair_rows_kernel(const bf16* gate_up, int rows, int ffn, bf
   }
 }
 
-// The same over eight features per thread (ffn a multiple of 8, 16-byte aligned rows): the prompt path's form.
-__global__ void silu_pair_rows_vec_kernel(const bf16* gate_up, int rows, int ffn, bf16* out) {
-  grid_dependency_wait();
-  const int per_row = ffn / 8;
-  const long long total = (long long)rows * per_row;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int row = int(i / per_row), n = int(i - (long long)row * per_row) * 8;
-    const uint4 g = *reinterpret_cast<const uint4*>(gate_up + size_t(row) * 2 * ffn + n);
-    const uint4 u = *reinterpret_cast<const uint4*>(gate_up + size_t(row) * 2 * ffn + ffn + n);
-    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
-    uint32_t packed[4];
-    // The branches for tiny and very negative gates are taken only where one of the eight needs them.
-    bool rare = false;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) rare |= silu_is_rare(bf16_lo(gw[j])) || silu_is_rare(bf16_hi(gw[j]));
-    if (rare) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        packed[j] = pack_bf16(silu_multiply_value(bf16_lo(gw[j]), bf16_lo(uw[j])),
-                              silu_multiply_value(bf16_hi(gw[j]), bf16_hi(uw[j])));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        packed[j] = pack_bf16(silu_multiply_common(bf16_lo(gw[j]), bf16_lo(uw[j])),
-                              silu_multiply_common(bf16_hi(gw[j]), bf16_hi(uw[j])));
-    }
-    *reinterpret_cast<uint4*>(out + size_t(row) * ffn + n) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-  }
-}
-
 // residual += projection (BF16, already rounded with bias), then RMSNorm: the unfused fallback of
 // launch_residual_norm for shapes the streaming GEMM does not take.
 __global__ void __launch_bounds__(512) residual_norm_bf16_kernel(const bf16* projection, int hidden, bf16* residual,
@@ -305,16 +275,11 @@ bool prompt_linear_ok(const PreparedLinear& w) {
          prompt_gemm_eligible(w.quantized, w.group_size, w.out, w.in, nullptr, w.in, nullptr, w.out);
 }
 
-// ksplit == 0: BF16 output with bias; otherwise FP32 partial sums of `ksplit` K slices in the workspace.
-void run_prompt_linear(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl,
-                       int ksplit, int x_stride, float* partial) {
+namespace {
+GemmParams prompt_params(const ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out) {
   GemmParams p{};
-  p.epilogue = ksplit ? kEpiPartial : kEpiStore;
-  p.ksplit = ksplit;
-  p.activation = w.activation;
-  p.partial = partial ? partial : s.model->prompt.partial;
   p.x = x;
-  p.x_stride = x_stride ? x_stride : w.in;
+  p.x_stride = w.in;
   p.M = rows;
   p.K = w.in;
   p.N = w.out;
@@ -329,6 +294,10 @@ void run_prompt_linear(ei_session& s, const PreparedLinear& w, const bf16* x, in
   p.out = out;
   p.out_stride = w.out;
   p.status = &s.control->status;
+  return p;
+}
+
+void enqueue_prompt_gemm(ei_session& s, const PreparedLinear& w, GemmParams& p, bool pdl) {
   if (s.inject_wait_polls) {
     p.wait_limit = s.inject_wait_polls;
     p.fault_tx = 16;
@@ -336,6 +305,29 @@ void run_prompt_linear(ei_session& s, const PreparedLinear& w, const bf16* x, in
   }
   tick(s);
   launch_prompt_gemm(w.quantized, p, s.stream, pdl);
+}
+}  // namespace
+
+// ksplit == 0: BF16 output with bias; otherwise FP32 partial sums of `ksplit` K slices in the workspace.
+void run_prompt_linear(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl,
+                       int ksplit, int x_stride, float* partial) {
+  GemmParams p = prompt_params(s, w, x, rows, out);
+  p.epilogue = ksplit ? kEpiPartial : kEpiStore;
+  p.ksplit = ksplit;
+  p.activation = w.activation;
+  p.partial = partial ? partial : s.model->prompt.partial;
+  if (x_stride) p.x_stride = x_stride;
+  enqueue_prompt_gemm(s, w, p, pdl);
+}
+
+// Gate and up projection (w: the gate's rows, then the up projection's) and the gated unit of their results in one launch.
+void run_prompt_gated(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl) {
+  GemmParams p = prompt_params(s, w, x, rows, out);
+  p.epilogue = kEpiSiluPair;
+  p.glu = w.glu;
+  p.glu_limit = w.glu_limit;
+  p.out_stride = w.out / 2;
+  enqueue_prompt_gemm(s, w, p, pdl);
 }
 
 // A projection with a BF16 output over all rows of a segment. Few output tiles (the q|k|v projection of a short
@@ -496,7 +488,7 @@ void ensure_prompt_workspace(ei_model& m) {
     return at;
   };
   const size_t o_residual = take(rows * H * 2), o_normed = take(rows * H * 2), o_qkv = take(rows * qkv_width * 2);
-  const size_t o_attention = take(rows * Q * 2), o_gate_up = take(rows * 2 * F * 2), o_act = take(rows * F * 2);
+  const size_t o_attention = take(rows * Q * 2), o_act = take(rows * F * 2);
   const size_t o_projection = take(rows * H * 2), o_tokens = take(rows * 4), o_step = take(rows * 4);
   // Room for the FP32 sums of a full segment, or for 16 K slices of a short one.
   const size_t partial_bytes = std::max(rows, size_t(16) * std::min<size_t>(rows, 256)) * H * sizeof(float);
@@ -511,7 +503,6 @@ void ensure_prompt_workspace(ei_model& m) {
   ws.normed = reinterpret_cast<bf16*>(base + o_normed);
   ws.qkv = reinterpret_cast<bf16*>(base + o_qkv);
   ws.attention = reinterpret_cast<bf16*>(base + o_attention);
-  ws.gate_up = reinterpret_cast<bf16*>(base + o_gate_up);
   ws.act = reinterpret_cast<bf16*>(base + o_act);
   ws.projection = reinterpret_cast<bf16*>(base + o_projection);
   ws.tokens = reinterpret_cast<uint32_t*>(base + o_tokens);
@@ -597,7 +588,6 @@ void enqueue_prompt_segment(ei_session& s, int rows, bool head) {
   tick(s);
   launch_embed_norm(e, s.stream, false);
 
-  const int elementwise_blocks = m.multiprocessors * 8;
   for (size_t layer = 0; layer < m.layers.size(); ++layer) {
     const auto& L = m.layers[layer];
     run_prompt_linear_store(s, L.qkv, ws.normed, rows, ws.qkv, pdl);
@@ -638,14 +628,7 @@ void enqueue_prompt_segment(ei_session& s, int rows, bool head) {
 
     run_prompt_projection_residual_norm(s, L.o, ws.attention, rows, L.ffn_norm, pdl);
 
-    run_prompt_linear(s, L.gate_up, ws.normed, rows, ws.gate_up, pdl);
-    tick(s);
-    if (ffn % 8 == 0)
-      launch(silu_pair_rows_vec_kernel, dim3(elementwise_blocks), dim3(256), 0, s.stream, pdl, (const bf16*)ws.gate_up,
-             rows, ffn, ws.act);
-    else
-      launch(silu_pair_rows_kernel, dim3(elementwise_blocks), dim3(256), 0, s.stream, pdl, (const bf16*)ws.gate_up, rows,
-             ffn, ws.act);
+    run_prompt_gated(s, L.gate_up, ws.normed, rows, ws.act, pdl);
     const bf16* next_norm = layer + 1 < m.layers.size() ? m.layers[layer + 1].attention_norm : m.output_norm;
     run_prompt_projection_residual_norm(s, L.down, ws.act, rows, next_norm, pdl);
   }
@@ -1031,14 +1014,7 @@ void enqueue_wide_batch_step(ei_batch& batch, int rows) {
     launch_verify_attention(a, lead.stream, pdl);
 
     run_prompt_projection_residual_norm(lead, L.o, ws.attention, total, L.ffn_norm, pdl);
-    run_prompt_linear(lead, L.gate_up, ws.normed, total, ws.gate_up, pdl);
-    tick(lead);
-    if (ffn % 8 == 0)
-      launch(silu_pair_rows_vec_kernel, dim3(m.multiprocessors * 8), dim3(256), 0, lead.stream, pdl,
-             (const bf16*)ws.gate_up, total, ffn, ws.act);
-    else
-      launch(silu_pair_rows_kernel, dim3(m.multiprocessors * 8), dim3(256), 0, lead.stream, pdl,
-             (const bf16*)ws.gate_up, total, ffn, ws.act);
+    run_prompt_gated(lead, L.gate_up, ws.normed, total, ws.act, pdl);
     const bf16* next_norm = layer + 1 < m.layers.size() ? m.layers[layer + 1].attention_norm : m.output_norm;
     run_prompt_projection_residual_norm(lead, L.down, ws.act, total, next_norm, pdl);
   }

@@ -65,8 +65,8 @@ struct ei_model {
     std::mutex mutex;
     unsigned char* arena = nullptr;
     size_t rows = 0;
-    ei::bf16 *residual = nullptr, *normed = nullptr, *qkv = nullptr, *attention = nullptr, *gate_up = nullptr,
-         *act = nullptr, *projection = nullptr;
+    ei::bf16 *residual = nullptr, *normed = nullptr, *qkv = nullptr, *attention = nullptr, *act = nullptr,
+         *projection = nullptr;
     float* partial = nullptr;         // FP32 sums of the o / down projections: [K slices][rows][hidden]
     size_t partial_bytes = 0;
     uint32_t *tokens = nullptr, *step_tokens = nullptr;
@@ -132,6 +132,8 @@ bool has_plan(const ei_session& s, const PreparedLinear& w, int rows, int epilog
 bool prompt_linear_ok(const PreparedLinear& w);
 void run_prompt_linear(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl,
                        int ksplit = 0, int x_stride = 0, float* partial = nullptr);
+// Gate and up projection and the gated unit of their BF16 results in one launch.
+void run_prompt_gated(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl);
 void run_prompt_linear_store(ei_session& s, const PreparedLinear& w, const bf16* x, int rows, bf16* out, bool pdl,
                              int x_stride = 0);
 // Commits all rows of a step. `folded`: the step's kernels already carried their recurrent state past these rows (a
