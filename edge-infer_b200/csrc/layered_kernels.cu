@@ -86,88 +86,138 @@ __global__ void __launch_bounds__(kJoinThreads) sublayer_join_kernel(const Subla
   }
 }
 
-// One warp per (row, unit); units in the order of the fused projection: q heads, k heads, v heads, then the linear
+// A unit is 256 bytes a row: a warp that takes one has a single load in flight and waits for it. A prompt's warps take four rows
+// of a unit (1500 rows of 80 units: the whole prompt 7.57 -> 7.44 ms, 14 launches), a step's up to 16 rows one each, so that
+// they fill the chip.
+// One warp per (kRows rows, unit); units in the order of the fused projection: q heads, k heads, v heads, then the linear
 // attention's q, k and v heads.
-template <typename T>
+template <typename T, int kRows>
 __global__ void __launch_bounds__(128) mixer_prepare_kernel(const MixerPrepareParams p) {
   const int warp = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int units = p.heads + 2 * p.kv_heads + 3 * p.lin_heads;
   const int context = p.control->context;  // written by the previous step
   grid_dependency_wait();
   grid_launch_dependents();
-  if (warp >= p.rows * units || context < 0 || context + p.rows > p.capacity) return;
-  const int row = warp / units;
-  int unit = warp - row * units;
-  const int position = context + row;
-  T* x = static_cast<T*>(p.fused) + size_t(row) * p.stride;
+  const int first_row = warp / units * kRows;
+  if (first_row >= p.rows || context < 0 || context + p.rows > p.capacity) return;
+  int unit = warp - warp / units * units;
+  // Row r of the warp, the last one again beyond the end (loaded, not stored).
+  int row_of[kRows];
+  bool live[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    live[r] = first_row + r < p.rows;
+    row_of[r] = live[r] ? first_row + r : p.rows - 1;
+  }
+  T* const fused = static_cast<T*>(p.fused);
 
   if (unit < p.heads + p.kv_heads) {  // rotation of a q or k head; k goes to the cache
     const bool key = unit >= p.heads;
-    x += size_t(unit) * p.dim_pad;
-    T* to = key ? static_cast<T*>(p.k_cache) + (size_t(position) * p.kv_heads + (unit - p.heads)) * p.dim_pad : x;
+    const T* x[kRows];
+    T* to[kRows];
+    const float2* turn[kRows];
     const int half = p.rot_dims >> 1;
-    const float2* turn = p.rotation + size_t(position) * half;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int position = context + row_of[r];
+      T* const own = fused + size_t(row_of[r]) * p.stride + size_t(unit) * p.dim_pad;
+      x[r] = own;
+      to[r] = key ? static_cast<T*>(p.k_cache) + (size_t(position) * p.kv_heads + (unit - p.heads)) * p.dim_pad : own;
+      turn[r] = p.rotation + size_t(position) * half;
+    }
     if (half % 4 == 0) {
       for (int i = lane * 4; i < half; i += 128) {
-        const float4 u = load_quad(x + i), v = load_quad(x + i + half);
-        const float4 t01 = *reinterpret_cast<const float4*>(turn + i), t23 = *reinterpret_cast<const float4*>(turn + i + 2);
-        store_quad(to + i, make_float4(u.x * t01.x - v.x * t01.y, u.y * t01.z - v.y * t01.w, u.z * t23.x - v.z * t23.y,
-                                       u.w * t23.z - v.w * t23.w));
-        store_quad(to + i + half, make_float4(v.x * t01.x + u.x * t01.y, v.y * t01.z + u.y * t01.w, v.z * t23.x + u.z * t23.y,
-                                              v.w * t23.z + u.w * t23.w));
-      }
-    } else if (half & 1) {
-      for (int i = lane; i < half; i += 32) {
-        const float u = value_of(x[i]), v = value_of(x[i + half]);
-        const float2 t = turn[i];
-        store_value(to + i, u * t.x - v * t.y);
-        store_value(to + i + half, v * t.x + u * t.y);
+        float4 u[kRows], v[kRows], t01[kRows], t23[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          u[r] = load_quad(x[r] + i);
+          v[r] = load_quad(x[r] + i + half);
+          t01[r] = *reinterpret_cast<const float4*>(turn[r] + i);
+          t23[r] = *reinterpret_cast<const float4*>(turn[r] + i + 2);
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          if (!live[r]) continue;
+          store_quad(to[r] + i, make_float4(u[r].x * t01[r].x - v[r].x * t01[r].y, u[r].y * t01[r].z - v[r].y * t01[r].w,
+                                            u[r].z * t23[r].x - v[r].z * t23[r].y, u[r].w * t23[r].z - v[r].w * t23[r].w));
+          store_quad(to[r] + i + half, make_float4(v[r].x * t01[r].x + u[r].x * t01[r].y, v[r].y * t01[r].z + u[r].y * t01[r].w,
+                                                   v[r].z * t23[r].x + u[r].z * t23[r].y, v[r].w * t23[r].z + u[r].w * t23[r].w));
+        }
       }
     } else {
-      for (int i = lane * 2; i < half; i += 64) {
-        const float2 u = load_pair(x + i), v = load_pair(x + i + half);
-        const float2 t0 = turn[i], t1 = turn[i + 1];
-        store_pair(to + i, u.x * t0.x - v.x * t0.y, u.y * t1.x - v.y * t1.y);
-        store_pair(to + i + half, v.x * t0.x + u.x * t0.y, v.y * t1.x + u.y * t1.y);
+      for (int r = 0; r < kRows && live[r]; ++r) {
+        if (half & 1) {
+          for (int i = lane; i < half; i += 32) {
+            const float u = value_of(x[r][i]), v = value_of(x[r][i + half]);
+            const float2 t = turn[r][i];
+            store_value(to[r] + i, u * t.x - v * t.y);
+            store_value(to[r] + i + half, v * t.x + u * t.y);
+          }
+        } else {
+          for (int i = lane * 2; i < half; i += 64) {
+            const float2 u = load_pair(x[r] + i), v = load_pair(x[r] + i + half);
+            const float2 t0 = turn[r][i], t1 = turn[r][i + 1];
+            store_pair(to[r] + i, u.x * t0.x - v.x * t0.y, u.y * t1.x - v.y * t1.y);
+            store_pair(to[r] + i + half, v.x * t0.x + u.x * t0.y, v.y * t1.x + u.y * t1.y);
+          }
+        }
       }
     }
     if (key)
       for (int i = p.rot_dims + lane * 2; i < p.dim_pad; i += 64) {
-        const float2 v = load_pair(x + i);
-        store_pair(to + i, v.x, v.y);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const float2 v = load_pair(x[r] + i);
+          if (live[r]) store_pair(to[r] + i, v.x, v.y);
+        }
       }
     return;
   }
   unit -= p.heads + p.kv_heads;
-  x += size_t(p.heads + p.kv_heads) * p.dim_pad;
+  size_t at = size_t(p.heads + p.kv_heads) * p.dim_pad;
   if (unit < p.kv_heads) {  // value norm, into the cache
-    x += size_t(unit) * p.vdim_pad;
-    T* to = static_cast<T*>(p.v_cache) + (size_t(position) * p.kv_heads + unit) * p.vdim_pad;
-    float sum = 0.0f;
+    at += size_t(unit) * p.vdim_pad;
+    float sum[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) sum[r] = 0.0f;
     for (int i = lane * 4; i < p.vdim_pad; i += 128) {
-      const float4 v = load_quad(x + i);
-      sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum))));
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const float4 v = load_quad(fused + size_t(row_of[r]) * p.stride + at + i);
+        sum[r] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum[r]))));
+      }
     }
-    const float inverse = 1.0f / sqrtf(warp_sum(sum) / float(p.vdim) + p.eps);
-    for (int i = lane * 4; i < p.vdim_pad; i += 128) {
-      const float4 v = load_quad(x + i);
-      store_quad(to + i, make_float4(v.x * inverse, v.y * inverse, v.z * inverse, v.w * inverse));
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const float inverse = 1.0f / sqrtf(warp_sum(sum[r]) / float(p.vdim) + p.eps);
+      if (!live[r]) continue;
+      T* const to = static_cast<T*>(p.v_cache) + (size_t(context + row_of[r]) * p.kv_heads + unit) * p.vdim_pad;
+      for (int i = lane * 4; i < p.vdim_pad; i += 128) {
+        const float4 v = load_quad(fused + size_t(row_of[r]) * p.stride + at + i);
+        store_quad(to + i, make_float4(v.x * inverse, v.y * inverse, v.z * inverse, v.w * inverse));
+      }
     }
     return;
   }
   unit -= p.kv_heads;
-  x += size_t(p.kv_heads) * p.vdim_pad;
+  at += size_t(p.kv_heads) * p.vdim_pad;
   const int kind = unit / p.lin_heads, head = unit - kind * p.lin_heads;  // 0 q, 1 k, 2 v
   const int pad = kind == 2 ? p.lin_vdim_pad : p.lin_dim_pad;
-  x += size_t(min(kind, 2)) * p.lin_heads * p.lin_dim_pad + size_t(head) * pad;
-  T* ring = nullptr;
-  if (p.ring_k && kind > 0)
-    ring = static_cast<T*>(kind == 1 ? p.ring_k : p.ring_v) + (size_t(position & (kRingRows - 1)) * p.lin_heads + head) * pad;
+  at += size_t(min(kind, 2)) * p.lin_heads * p.lin_dim_pad + size_t(head) * pad;
   for (int i = lane * 4; i < pad; i += 128) {
-    float4 v = load_quad(x + i);
-    v = make_float4(silu_for<T>(v.x), silu_for<T>(v.y), silu_for<T>(v.z), silu_for<T>(v.w));
-    store_quad(x + i, v);
-    if (ring) store_quad(ring + i, v);
+    float4 v[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) v[r] = load_quad(fused + size_t(row_of[r]) * p.stride + at + i);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      if (!live[r]) continue;
+      const float4 y = make_float4(silu_for<T>(v[r].x), silu_for<T>(v[r].y), silu_for<T>(v[r].z), silu_for<T>(v[r].w));
+      store_quad(fused + size_t(row_of[r]) * p.stride + at + i, y);
+      if (p.ring_k && kind > 0) {
+        T* const ring = static_cast<T*>(kind == 1 ? p.ring_k : p.ring_v);
+        store_quad(ring + (size_t((context + row_of[r]) & (kRingRows - 1)) * p.lin_heads + head) * pad + i, y);
+      }
+    }
   }
 }
 
@@ -505,8 +555,11 @@ void launch_sublayer_join(const SublayerJoinParams& p, cudaStream_t stream, bool
 }
 template <typename T>
 void launch_mixer_prepare(const MixerPrepareParams& p, cudaStream_t stream, bool pdl) {
-  const int warps = p.rows * (p.heads + 2 * p.kv_heads + 3 * p.lin_heads);
-  launch(mixer_prepare_kernel<T>, dim3(unsigned((warps + 3) / 4)), dim3(128), 0, stream, pdl, p);
+  const int units = p.heads + 2 * p.kv_heads + 3 * p.lin_heads;
+  if (p.rows > kMaxRows)
+    launch(mixer_prepare_kernel<T, 4>, dim3(unsigned(((p.rows + 3) / 4 * units + 3) / 4)), dim3(128), 0, stream, pdl, p);
+  else
+    launch(mixer_prepare_kernel<T, 1>, dim3(unsigned((p.rows * units + 3) / 4)), dim3(128), 0, stream, pdl, p);
 }
 template <typename T>
 void launch_mixer_finish(const MixerFinishParams& p, cudaStream_t stream, bool pdl) {
