@@ -28,12 +28,17 @@ constexpr int kDim = 128;
 constexpr int kPartial = 132;      // floats per (split, row, head): 128 outputs, m, l, padding
 constexpr int kTileBytes = kTile * kDim * 2;
 
-constexpr int kStages = 3;                     // K/V tiles in flight per block
-constexpr int kStageBytes = 2 * kTileBytes;    // one K tile and one V tile
-constexpr size_t kAttentionShared = size_t(kStages) * kStageBytes + 1024 /* alignment */ + 64;
+// The ring: K and V tiles in turn, a buffer each. A block of several warps has four buffers, two tiles; two such blocks share an
+// SM (registers). A block of one warp knows without a barrier that K has been read, hands K's buffer on as soon as the scores
+// stand and gets by on three, so that four blocks share an SM. What bounds those is the chain of one warp, 2 us a tile, at two
+// blocks on an SM (rings of three tiles, 97 KB) 0.66 of the HBM peak: 64 splits of 8 KV heads were two waves, now they are one.
+// Steps, three tiles a block -> this: 8B int4, 4 rows behind 30 000 tokens 2.92 -> 2.72 ms, 9 rows behind 2000 2.583 -> 2.566,
+// 64 x 5 rows of 7B int4 9.34 -> 9.24; 1.7B and 0.6B the same. (Two tiles, so that three one-warp blocks share an SM: 3.03 at
+// the first size, where 28 of 472 blocks make a second wave that costs almost as much as the first.)
+constexpr size_t attention_shared(int buffers) { return size_t(buffers) * kTileBytes + 1024 /* alignment */ + 64; }
 
 struct AttentionShared {
-  uint64_t full[kStages];
+  uint64_t full[2];  // by tile, of either parity
   int failed;
 };
 
@@ -45,11 +50,12 @@ __device__ __forceinline__ int tile_offset(int token, int chunk) {
 
 // Block (split, kv head) covers one chunk of the sequence for all <= 16 query rows and writes (o, m, l) partials for the
 // merge kernel.
-__global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_constant__ AttentionParams p) {
+template <int kBuffers>
+__global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_kernel(const __grid_constant__ AttentionParams p) {
   extern __shared__ unsigned char attention_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(attention_smem_raw) + 1023) &
                                                          ~uintptr_t(1023));
-  AttentionShared* sh = reinterpret_cast<AttentionShared*>(smem + size_t(kStages) * kStageBytes);
+  AttentionShared* sh = reinterpret_cast<AttentionShared*>(smem + size_t(kBuffers) * kTileBytes);
   // The context length was written by the previous step; the preceding kernel of this step only appends the
   // new rows [offset, offset + rows). A chunk that ends before them can start fetching at once.
   // Wide batch (split form only): grid slice z is a session with its own cache, context length, queries, scratch.
@@ -84,24 +90,30 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   const int tiles = (end - start + kTile - 1) / kTile;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) mbarrier_init(&sh->full[s], 1);
+    for (int b = 0; b < 2; ++b) mbarrier_init(&sh->full[b], 1);
     sh->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // One thread requests a tile: the K and the V box of 64 tokens of this KV head, one stage of the ring.
-  auto request = [&](int tile) {
-    const int stage = tile % kStages;
-    unsigned char* base = smem + size_t(stage) * kStageBytes;
-    mbarrier_expect_tx(&sh->full[stage], uint32_t(kStageBytes) + (tile == 0 ? p.fault_tx : 0u));
-    tma_load_5d(base, k_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[stage]);
-    tma_load_5d(base + kTileBytes, v_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[stage]);
+  // One thread requests the boxes of 64 tokens of this KV head. K's arms the tile's barrier for both.
+  auto request_keys = [&](int tile, int buffer) {
+    if (tile >= tiles) return;
+    mbarrier_expect_tx(&sh->full[tile & 1], uint32_t(2 * kTileBytes) + (tile == 0 ? p.fault_tx : 0u));
+    tma_load_5d(smem + buffer * kTileBytes, k_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile & 1]);
+  };
+  auto request_values = [&](int tile, int buffer) {
+    if (tile >= tiles) return;
+    tma_load_5d(smem + buffer * kTileBytes, v_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile & 1]);
   };
 
   const bool settled = end <= offset;  // no row of this chunk is written by the preceding kernel
   if (!settled) grid_dependency_wait();
-  if (threadIdx.x == 0)
-    for (int tile = 0; tile < min(kStages, tiles); ++tile) request(tile);
+  if (threadIdx.x == 0) {
+    request_keys(0, 0);
+    request_values(0, 1);
+    request_keys(1, 2);
+    if (kBuffers == 4) request_values(1, 3);
+  }
   if (settled) grid_dependency_wait();  // the queries come from the preceding kernel
   // Only now: a kernel that triggers after its own wait lets its successor's prologue see everything up to the
   // kernel before this one as complete, which is what the early fetch above relies on.
@@ -134,13 +146,13 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
   for (int d = 0; d < 16; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.0f;
   float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.0f, l_hi = 0.0f;
 
-  int tile = 0;
+  int tile = 0, keys = 0;  // the tile, the buffer of its K
   bool gave_up = false;
   for (; tile < tiles; ++tile) {
-    const int stage = tile % kStages;
-    if (!mbarrier_wait(&sh->full[stage], (tile / kStages) & 1, wait_limit)) sh->failed = 1;
-    unsigned char* ks = smem + size_t(stage) * kStageBytes;
-    unsigned char* vs = ks + kTileBytes;
+    if (!mbarrier_wait(&sh->full[tile & 1], (tile >> 1) & 1, wait_limit)) sh->failed = 1;
+    const int values = keys + 1 == kBuffers ? 0 : keys + 1;
+    unsigned char* ks = smem + keys * kTileBytes;
+    unsigned char* vs = smem + values * kTileBytes;
     const int first = start + tile * kTile;
     const bool masked = first + kTile - 1 > offset;
     if (end - first < kTile) {
@@ -194,6 +206,9 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
     new_lo = fmaxf(new_lo, __shfl_xor_sync(0xffffffffu, new_lo, 2));
     new_hi = fmaxf(new_hi, __shfl_xor_sync(0xffffffffu, new_hi, 1));
     new_hi = fmaxf(new_hi, __shfl_xor_sync(0xffffffffu, new_hi, 2));
+    // One warp, whose lanes all have their scores here (the maxima come of them): K's buffer takes the next tile's V. Also
+    // where this tile's wait ran out: that V belongs to the next tile's barrier, which its K has armed.
+    if (kBuffers == 3 && threadIdx.x == 0) request_values(tile + 1, keys);
     // A row with nothing visible yet keeps m = -inf; use 0 as the exponent base so that the power is 0.
     const float top_lo = new_lo == -INFINITY ? 0.0f : new_lo, top_hi = new_hi == -INFINITY ? 0.0f : new_hi;
     const float base_lo = top_lo * exponent_scale, base_hi = top_hi * exponent_scale;
@@ -243,14 +258,18 @@ __global__ void __launch_bounds__(224) verify_attention_kernel(const __grid_cons
     __syncthreads();  // every warp is done with this stage
     gave_up = sh->failed != 0;  // written before the barrier by any thread whose wait ran out: block-uniform
     if (gave_up) break;
-    if (threadIdx.x == 0 && tile + kStages < tiles) request(tile + kStages);
+    if (threadIdx.x == 0) {
+      request_keys(tile + 2, kBuffers == 4 ? keys : values);
+      if (kBuffers == 4) request_values(tile + 2, values);
+    }
+    keys = keys >= 2 ? keys + 2 - kBuffers : keys + 2 == kBuffers ? 0 : 2;
   }
   if (gave_up) {
     // Copies still in flight write into this block's shared memory: wait for them (bounded) before leaving. The
     // copy of tile 0 carries the test hook's unmet expectation when that is armed and is known not to complete.
     if (threadIdx.x == 0) {
-      for (int t = max(tile, p.fault_tx ? 1 : 0); t < min(tile + kStages, tiles); ++t)
-        mbarrier_wait(&sh->full[t % kStages], (t / kStages) & 1, wait_limit);
+      for (int t = max(tile, p.fault_tx ? 1 : 0); t < min(tile + 2, tiles); ++t)
+        mbarrier_wait(&sh->full[t & 1], (t >> 1) & 1, wait_limit);
       if (p.status) atomicOr(p.status, 4);
     }
     return;
@@ -480,8 +499,8 @@ void configure_attention_kernels() {
   int device = 0;
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device == device) return;
-  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(kAttentionShared)));
+  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attention_shared(3))));
+  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attention_shared(4))));
   EI_CUDA(cudaFuncSetAttribute(prompt_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PaLayout<kDim>::kTotal)));
   configured_device = device;
 }
@@ -517,8 +536,10 @@ void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool
   configure_attention_kernels();
   const AttentionParams q = with_maps(p);
   const unsigned sessions = q.slots ? unsigned(q.sessions) : 1u;
-  launch(verify_attention_kernel, dim3(q.kv_heads, q.max_splits, sessions), dim3(warps * 32), kAttentionShared,
-         stream, pdl, q);
+  // One warp: three buffers, four blocks on an SM; more: registers allow two blocks, which may as well hold two tiles.
+  const int buffers = warps == 1 ? 3 : 4;
+  launch(warps == 1 ? verify_attention_kernel<3> : verify_attention_kernel<4>, dim3(q.kv_heads, q.max_splits, sessions),
+         dim3(warps * 32), attention_shared(buffers), stream, pdl, q);
   if (q.slots && !q.merge_blocks)
     launch(attention_merge_wide_kernel, dim3((q.rows * q.heads * q.sessions + 3) / 4), dim3(128), 0, stream, pdl, q);
   else
