@@ -7,8 +7,11 @@
 namespace ei {
 namespace {
 
-constexpr int kHeld = 4;  // quads of a row a thread keeps in registers; the rest is read again
-constexpr int kMostThreads = 1024;
+// Quads of a row that a thread keeps in registers (the rest is read again): four in the blocks of 256 that many rows get, one in
+// a step's blocks of up to 512 or 1024, which have a thread for every quad. (One kernel for all, of 64 registers a thread and
+// four quads, spilled 220 bytes: 2048 rows through 28 layers 10.16 -> 10.07 ms, a step at width 1024 864 -> 856 us.)
+constexpr int kMostThreads = 1024, kStepThreads = 512, kManyRowThreads = 256;
+constexpr int held_quads(int threads) { return threads == kManyRowThreads ? 4 : 1; }
 
 __device__ __forceinline__ float masked_sum(float4 x, int i, int width) {
   return (i < width ? x.x : 0.0f) + (i + 1 < width ? x.y : 0.0f) + (i + 2 < width ? x.z : 0.0f) + (i + 3 < width ? x.w : 0.0f);
@@ -31,7 +34,7 @@ __device__ __forceinline__ FirstWeights first_weights(const RowNorms& n, int col
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   return {i < columns ? load_quad(n.first + i) : zero, i < columns && n.second ? load_quad(n.second + i) : zero};
 }
-template <typename T>
+template <typename T, int kHeld>
 __device__ __forceinline__ void norm_row(const RowNorms& n, const float4 (&held)[kHeld], const float* residual, int columns,
                                          int row, float* shared, const FirstWeights& ahead) {
   const int step = blockDim.x * 4;
@@ -64,8 +67,9 @@ __device__ __forceinline__ void norm_row(const RowNorms& n, const float4 (&held)
     emit(i, i < columns ? *reinterpret_cast<const float4*>(residual + i) : zero);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kMostThreads) parallel_embed_kernel(const ParallelEmbedParams p) {
+template <typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads) parallel_embed_kernel(const ParallelEmbedParams p) {
+  constexpr int kHeld = held_quads(kThreads);
   __shared__ uint32_t token_shared;
   __shared__ unsigned long long pair_shared;
   __shared__ float shared[2 * kMostThreads / 32];
@@ -105,11 +109,12 @@ __global__ void __launch_bounds__(kMostThreads) parallel_embed_kernel(const Para
     held[j] = i < p.residual_stride ? fetch(i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   for (int i = (threadIdx.x + kHeld * blockDim.x) * 4; i < p.residual_stride; i += blockDim.x * 4) fetch(i);
-  norm_row<T>(p.norms, held, residual, p.residual_stride, row, shared, ahead);
+  norm_row<T, kHeld>(p.norms, held, residual, p.residual_stride, row, shared, ahead);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kMostThreads) parallel_join_kernel(const ParallelJoinParams p) {
+template <typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads) parallel_join_kernel(const ParallelJoinParams p) {
+  constexpr int kHeld = held_quads(kThreads);
   __shared__ float shared[2 * kMostThreads / 32];
   // Weights do not come from the preceding kernel.
   const FirstWeights ahead = first_weights(p.norms, p.residual_stride);
@@ -154,24 +159,32 @@ __global__ void __launch_bounds__(kMostThreads) parallel_join_kernel(const Paral
     held[j] = i < p.residual_stride ? join(i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   for (int i = (threadIdx.x + kHeld * blockDim.x) * 4; i < p.residual_stride; i += blockDim.x * 4) join(i);
-  norm_row<T>(p.norms, held, residual, p.residual_stride, row, shared, ahead);
+  norm_row<T, kHeld>(p.norms, held, residual, p.residual_stride, row, shared, ahead);
 }
 
 // A few rows: one quad per thread as far as a block goes. Many: blocks of 256.
 unsigned row_threads(int rows, int stride) {
   const int whole = (stride / 4 + 31) / 32 * 32;
-  return unsigned(std::min(whole, rows <= kMaxRows ? kMostThreads : 256));
+  return unsigned(std::min(whole, rows <= kMaxRows ? kMostThreads : kManyRowThreads));
 }
 
 }  // namespace
 
 template <typename T>
 void launch_parallel_embed(const ParallelEmbedParams& p, cudaStream_t stream, bool pdl) {
-  launch(parallel_embed_kernel<T>, dim3(unsigned(p.token.rows)), dim3(row_threads(p.token.rows, p.norms.stride)), 0, stream, pdl, p);
+  const unsigned threads = row_threads(p.token.rows, p.norms.stride);
+  launch(p.token.rows > kMaxRows    ? parallel_embed_kernel<T, kManyRowThreads>
+         : threads <= kStepThreads ? parallel_embed_kernel<T, kStepThreads>
+                                   : parallel_embed_kernel<T, kMostThreads>,
+         dim3(unsigned(p.token.rows)), dim3(threads), 0, stream, pdl, p);
 }
 template <typename T>
 void launch_parallel_join(const ParallelJoinParams& p, cudaStream_t stream, bool pdl) {
-  launch(parallel_join_kernel<T>, dim3(unsigned(p.rows)), dim3(row_threads(p.rows, p.norms.stride)), 0, stream, pdl, p);
+  const unsigned threads = row_threads(p.rows, p.norms.stride);
+  launch(p.rows > kMaxRows          ? parallel_join_kernel<T, kManyRowThreads>
+         : threads <= kStepThreads ? parallel_join_kernel<T, kStepThreads>
+                                   : parallel_join_kernel<T, kMostThreads>,
+         dim3(unsigned(p.rows)), dim3(threads), 0, stream, pdl, p);
 }
 template void launch_parallel_embed<bf16>(const ParallelEmbedParams&, cudaStream_t, bool);
 template void launch_parallel_embed<float>(const ParallelEmbedParams&, cudaStream_t, bool);
