@@ -172,7 +172,7 @@ void encode_kv_map(CUtensorMap* map, const bf16* base, size_t tokens, size_t tok
 int attention_chunk_for(size_t kv_length);
 size_t attention_scratch_bytes(size_t rows, size_t heads, size_t kv_length);
 void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool pdl);
-// Any number of query rows in one launch, 16 per block over their whole causal history; no scratch, no merge
+// Any number of query rows in one launch, up to 256 stacked ones per block over their whole causal history; no scratch, no merge
 // (chunk, max_splits and scratch are not used).
 void launch_prompt_attention(const AttentionParams& p, cudaStream_t stream, bool pdl);
 

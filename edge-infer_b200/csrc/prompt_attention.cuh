@@ -52,17 +52,6 @@ struct PaShared {
   int issued, query_tiles;            // tiles of keys and values, of queries whose copies were requested
 };
 
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_b, uint32_t desc_high, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 b, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
-      :
-      : "r"(tmem_d), "r"(tmem_a), "r"(desc_b), "r"(desc_high), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // 16 columns of the warp's 32 lanes, without waiting for them.
 __device__ __forceinline__ void tmem_request16(uint32_t address, uint32_t (&r)[16]) {
   asm volatile(
@@ -79,15 +68,6 @@ __device__ __forceinline__ void tmem_loaded(uint32_t (&r)[16]) {
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
                  "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
-__device__ __forceinline__ void tmem_store16(uint32_t address, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(address)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_stored() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // Two FP32 operations in one instruction.
 __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
   uint64_t r;

@@ -16,6 +16,7 @@ constexpr int kPromptWorkerWarps = 16;
 constexpr int kPromptTeamWarps = 4;    // int4: a team of warps dequantises a K block of the one feature tile
 constexpr int kPromptWeightBytes = kPromptFeatures * kPromptBlockK * 2;             // 16 KiB BF16 operand per feature tile
 constexpr int kPromptRawBytes = kPromptFeatures * (kPromptBlockK / 2);              // 4 KiB of int4 per feature tile
+constexpr int kPromptWeightColumns = kPromptBlockK / 2;  // of tensor memory, for the int4 operand of a K block
 constexpr size_t kPromptSharedExtra = 1024 /* alignment */ + 512;
 constexpr size_t kPromptSharedLimit = 227 * 1024;
 
@@ -24,12 +25,13 @@ struct PromptTile {
   int feature_tiles, token_tiles, columns;
   int x_stages, w_stages;  // K blocks of activations and of BF16 weights in the rings (x_stages >= w_stages)
   int raw_stages;          // int4: K blocks of packed weights; a multiple of w_stages
+  bool tensor_operands = false;  // int4: the dequantised weights stand in tensor memory, not in shared memory
 };
 
 // Bytes of the rings: activations, weight operands, packed int4 weights (every stage a multiple of 1024).
 constexpr int prompt_ring_bytes(const PromptTile& t) {
   return t.x_stages * t.token_tiles * t.columns * kPromptBlockK * 2 +
-         t.feature_tiles * (t.w_stages * kPromptWeightBytes + t.raw_stages * kPromptRawBytes);
+         t.feature_tiles * ((t.tensor_operands ? 0 : t.w_stages * kPromptWeightBytes) + t.raw_stages * kPromptRawBytes);
 }
 
 // The best shape of a launch and what it is estimated to cost, in SM cycles.
@@ -58,6 +60,24 @@ inline bool prompt_rings(bool awq, PromptTile& t) {
         if (t.x_stages >= std::max(wanted, t.w_stages)) return true;
       }
   return false;
+}
+
+// An int4 tile with its operands in the columns of tensor memory that the accumulators leave, where those are enough for two, and
+// the rings as deep as the shared memory so freed allows. Up to 448 tokens; 480 keep theirs in shared memory.
+inline PromptTile prompt_tensor_operands(const PromptTile& tile) {
+  PromptTile t = tile;
+  t.tensor_operands = true;
+  const int room = int(kPromptSharedLimit - kPromptSharedExtra), tokens = t.token_tiles * t.columns;
+  for (t.w_stages = kPromptWorkerWarps / kPromptTeamWarps; t.w_stages >= 2; --t.w_stages) {
+    if (tokens + t.w_stages * kPromptWeightColumns > kPromptTmemColumns) continue;
+    for (int rounds = 2; rounds >= 1; --rounds) {
+      t.raw_stages = rounds * t.w_stages;
+      t.x_stages = 0;
+      t.x_stages = std::min(kPromptMaxStages, (room - prompt_ring_bytes(t)) / (tokens * kPromptBlockK * 2));
+      if (t.x_stages >= std::max(t.w_stages, tile.x_stages)) return t;
+    }
+  }
+  return tile;
 }
 
 // The shapes considered for a problem, each with what its estimate needs at any K split: searched once and compared at every

@@ -28,14 +28,10 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device != device) {
     EI_CUDA(cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kPromptSharedLimit)));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kPromptSharedLimit)));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kPromptSharedLimit)));
-    EI_CUDA(cudaFuncSetAttribute(prompt_gemm_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kPromptSharedLimit)));
+    for (const auto kernel : {prompt_gemm_kernel<true, false, false>, prompt_gemm_kernel<true, false, true>,
+                              prompt_gemm_kernel<true, true, false>, prompt_gemm_kernel<true, true, true>,
+                              prompt_gemm_kernel<false, false, false>, prompt_gemm_kernel<false, true, false>})
+      EI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPromptSharedLimit)));
     configured_device = device;
   }
   const int ksplit = p.epilogue == kEpiPartial ? std::max(1, p.ksplit) : 1;
@@ -48,6 +44,7 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   GemmParams q = p;
   q.ksplit = ksplit;
   q.prompt = PromptShapes(awq, p.M, p.N, p.K, multiprocessors, gated).best(ksplit, p.epilogue == kEpiPartial, false).tile;
+  if (awq) q.prompt = prompt_tensor_operands(q.prompt);
   PromptMaps maps{};
   {
     const cuuint64_t dims[2] = {cuuint64_t(p.K), cuuint64_t(p.M)};
@@ -74,8 +71,10 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   const int tokens = q.prompt.token_tiles * q.prompt.columns, features = kPromptFeatures * q.prompt.feature_tiles;
   const size_t shared = size_t(prompt_ring_bytes(q.prompt)) + kPromptSharedExtra;
   const dim3 grid((p.N + features - 1) / features, (p.M + tokens - 1) / tokens, ksplit);
-  const auto kernel = awq ? (gated ? prompt_gemm_kernel<true, true> : prompt_gemm_kernel<true, false>)
-                          : (gated ? prompt_gemm_kernel<false, true> : prompt_gemm_kernel<false, false>);
+  const bool tensor = q.prompt.tensor_operands;
+  const auto kernel = !awq    ? (gated ? prompt_gemm_kernel<false, true, false> : prompt_gemm_kernel<false, false, false>)
+                      : gated ? (tensor ? prompt_gemm_kernel<true, true, true> : prompt_gemm_kernel<true, true, false>)
+                              : (tensor ? prompt_gemm_kernel<true, false, true> : prompt_gemm_kernel<true, false, false>);
   launch(kernel, grid, dim3(kPromptThreads), shared, stream, pdl, maps, q);
 }
 

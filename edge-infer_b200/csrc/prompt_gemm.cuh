@@ -18,10 +18,13 @@
 //     tcgen05.mma), BF16 weights as [128 features][64 inputs] swizzled boxes, int4 weights as raw [128 rows][32 bytes]
 //     boxes. The weights of the ring's first round are requested before the kernel waits for its predecessor, which does
 //     not write them;
-//   * for int4, teams of four of warps 0-15 turn the raw boxes into the BF16 K-major swizzled operand in shared memory,
-//     team j of w_stages every w_stages-th K block, with the exact dequantisation of the small-M kernels (dequant_pair:
-//     round_bf16((w - z) * scale)), fence the writes towards the asynchronous proxy and arrive on the K block's `ready`
-//     barrier;
+//   * for int4, teams of four of warps 0-15 turn the raw boxes into the BF16 operand, a row per lane of tensor memory, in the
+//     columns that the accumulators leave: team j of w_stages every w_stages-th K block, with the exact dequantisation of the
+//     small-M kernels (dequant_pair: round_bf16((w - z) * scale)); they arrive on the K block's `ready` barrier when their
+//     stores have completed. Shared memory is what a K block of many tokens is bound by (activations in, operands out): an
+//     operand in shared memory cost 128 cycles of stores (twice that while rows r and r + 4 met in a bank) and 32 a MMA of
+//     loads. 8B int4, 2048 rows: 30.4 ms with the conflict, 29.2 without, 28.5 from tensor memory; batches of 64 x 5 rows, 7B
+//     int4: 9.45, 9.40, 9.24;
 //   * one warp or, with more than one accumulator, two (warps 17 and 18) issue, per K block, feature tile and token
 //     tile, four tcgen05.mma (M 128, N columns, K 16) that accumulate in tensor memory, and commit the K block's `empty`
 //     barrier, which hands both operands' buffers back;
@@ -42,6 +45,7 @@
 // and the pairs' way out and back (6 us at 333 x 12288, 25-37 us at 2048 x 24576); in the epilogue, which nothing overlaps, the
 // units take 23 us of the latter's 305. Whole prompts, separate -> here: 1.7B, 333 rows 2.31 -> 2.18 ms; 8B int4, 2048 rows
 // 30.8 -> 30.5; 1500 rows of the 2048-wide join decoder 8.02 -> 7.67; a batch of 64 x 5 rows, 7B int4 9.80 -> 9.57.
+// (An int4 tile of 480 tokens leaves no columns: its operands stand in shared memory, swizzled, K-major, as BF16 ones do.)
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
 //
 // Every wait on an mbarrier is bounded. A role whose wait runs out raises a flag in shared memory that every
@@ -119,6 +123,28 @@ __device__ __forceinline__ void tmem_load16(uint32_t address, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+
+// The same with A in tensor memory: a row per lane, two inputs per column.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_b, uint32_t desc_high, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "r"(desc_b), "r"(desc_high), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_store16(uint32_t address, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::
+          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(address)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_stored() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_load8(uint32_t address, float (&v)[8]) {
   uint32_t r[8];
@@ -236,7 +262,7 @@ __device__ __forceinline__ void gated_units(int glu, float limit, uint32_t (&gat
   }
 }
 
-template <bool kAwq, bool kGated>
+template <bool kAwq, bool kGated, bool kTensorOperands>
 __global__ void __launch_bounds__(kPromptThreads, 1)
     prompt_gemm_kernel(const __grid_constant__ PromptMaps maps, const GemmParams p) {
   extern __shared__ unsigned char prompt_smem_raw[];
@@ -283,7 +309,8 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   const int raw_bytes = p.prompt.feature_tiles * kPromptRawBytes;
   unsigned char* const x_ring = smem;
   unsigned char* const w_ring = x_ring + p.prompt.x_stages * x_bytes;
-  unsigned char* const raw_ring = w_ring + p.prompt.w_stages * w_bytes;
+  unsigned char* const raw_ring = kTensorOperands ? w_ring : w_ring + p.prompt.w_stages * w_bytes;
+  const uint32_t w_tmem = tmem + kPromptTmemColumns - p.prompt.w_stages * kPromptWeightColumns;  // int4: the operands
 
   if (warp == kPromptWorkerWarps || warp == kPromptWorkerWarps + 3) {
     // ---- copy threads: one for the weights, one for the activations ----
@@ -345,12 +372,18 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
       const uint32_t instruction = prompt_instruction(columns);
       const int live = feature_tiles * token_tiles, second = mine + issuers;  // at most two accumulators per warp
       const int f0 = mine / token_tiles, m0 = mine - f0 * token_tiles, f1 = second / token_tiles, m1 = second - f1 * token_tiles;
-      const uint32_t a0 = umma_desc_low(smem_address(w_ring) + f0 * kPromptWeightBytes);
+      const uint32_t a0 = kTensorOperands ? w_tmem : umma_desc_low(smem_address(w_ring) + f0 * kPromptWeightBytes);
       const uint32_t b0 = umma_desc_low(smem_address(x_ring) + m0 * tile_bytes);
-      const uint32_t a1 = umma_desc_low(smem_address(w_ring) + f1 * kPromptWeightBytes);
+      const uint32_t a1 = kTensorOperands ? w_tmem : umma_desc_low(smem_address(w_ring) + f1 * kPromptWeightBytes);
       const uint32_t b1 = umma_desc_low(smem_address(x_ring) + m1 * tile_bytes);
       const uint32_t d0 = tmem + f0 * block_tokens + m0 * columns, d1 = tmem + f1 * block_tokens + m1 * columns;
-      const uint32_t w_step = uint32_t(w_bytes) >> 4, x_step = uint32_t(x_bytes) >> 4;
+      const uint32_t w_step = kTensorOperands ? kPromptWeightColumns : uint32_t(w_bytes) >> 4, x_step = uint32_t(x_bytes) >> 4;
+      auto multiply = [&](uint32_t d, uint32_t a, uint32_t b, int j, uint32_t accumulate) {
+        if (kTensorOperands)
+          umma_bf16_ts(d, a + j * 8, b + j * 2, kUmmaDescHigh, instruction, accumulate);
+        else
+          umma_bf16_ss(d, a + j * 2, b + j * 2, kUmmaDescHigh, instruction, accumulate);
+      };
       int w_slot = 0, slot = 0;
       uint32_t parity = 0, w_at = 0, x_at = 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
@@ -360,12 +393,12 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
           if (mine < live) {
 #pragma unroll
             for (int j = 0; j < kPromptBlockK / 16; ++j)  // 16 inputs = 32 bytes further along the swizzled row
-              umma_bf16_ss(d0, a0 + w_at + j * 2, b0 + x_at + j * 2, kUmmaDescHigh, instruction, j > 0 ? 1u : uint32_t(kb));
+              multiply(d0, a0 + w_at, b0 + x_at, j, j > 0 ? 1u : uint32_t(kb));
           }
           if (second < live) {
 #pragma unroll
             for (int j = 0; j < kPromptBlockK / 16; ++j)
-              umma_bf16_ss(d1, a1 + w_at + j * 2, b1 + x_at + j * 2, kUmmaDescHigh, instruction, j > 0 ? 1u : uint32_t(kb));
+              multiply(d1, a1 + w_at, b1 + x_at, j, j > 0 ? 1u : uint32_t(kb));
           }
           tcgen05_commit(&sh->empty[slot]);
         }
@@ -404,8 +437,10 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
       };
       const int end = team < teams ? k_blocks : 0;
       if (team < end) request(team);
-      unsigned char* const operand = w_ring + team * w_bytes + row * 128;
-      // Rows 4-7 of eight read their halves in the other order: the eight lanes of a load hit distinct banks.
+      const uint32_t operand = w_tmem + team * kPromptWeightColumns + (uint32_t(warp & 3) * 32 << 16);
+      unsigned char* const operand_row = w_ring + team * w_bytes + row * 128;
+      // Rows 4-7 of eight read their halves in the other order, so that the eight lanes of a load hit distinct banks, and change
+      // them back in registers.
       const unsigned char* const raw_row = raw_ring + row * 32;
       const int first_half = (row & 4) * 4;
       // K block kb takes the operand buffer that K block kb - teams leaves; the MMAs complete in order and the ring of
@@ -420,7 +455,9 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
         if (!__all_sync(0xffffffffu, prompt_wait(sh, &sh->raw_full[raw_slot], raw_parity, limit))) break;
         const uint4 raw0 = *reinterpret_cast<const uint4*>(raw_row + raw_slot * raw_bytes + first_half);
         const uint4 raw1 = *reinterpret_cast<const uint4*>(raw_row + raw_slot * raw_bytes + 16 - first_half);
-        const uint32_t words[8] = {raw0.x, raw0.y, raw0.z, raw0.w, raw1.x, raw1.y, raw1.z, raw1.w};
+        const bool second = row & 4;  // the second half came first
+        const uint32_t words[8] = {second ? raw1.x : raw0.x, second ? raw1.y : raw0.y, second ? raw1.z : raw0.z, second ? raw1.w : raw0.w,
+                                   second ? raw0.x : raw1.x, second ? raw0.y : raw1.y, second ? raw0.z : raw1.z, second ? raw0.w : raw1.w};
         if (kb != team) {  // the buffer is fresh in the team's first round
           if (!__all_sync(0xffffffffu, prompt_wait(sh, &sh->empty[left_slot], left_parity, limit))) break;
           left_slot += teams;
@@ -429,21 +466,38 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
             left_parity ^= 1;
           }
         }
+        if (kTensorOperands) tcgen05_fence_after();
 #pragma unroll
-        for (int w = 0; w < 8; ++w) {
-          // dequant_pair gives (k, k + 4) pairs; the operand wants the eight inputs of a word in order.
-          const uint32_t p0 = dequant_pair(words[w], zero2, scale2);
-          const uint32_t p1 = dequant_pair(words[w] >> 4, zero2, scale2);
-          const uint32_t p2 = dequant_pair(words[w] >> 8, zero2, scale2);
-          const uint32_t p3 = dequant_pair(words[w] >> 12, zero2, scale2);
-          uint4 o;
-          o.x = __byte_perm(p0, p1, 0x5410);
-          o.y = __byte_perm(p2, p3, 0x5410);
-          o.z = __byte_perm(p0, p1, 0x7632);
-          o.w = __byte_perm(p2, p3, 0x7632);
-          *reinterpret_cast<uint4*>(operand + ((w ^ (row & 4) ^ (row & 7)) << 4)) = o;
+        for (int half = 0; half < 2; ++half) {
+          uint32_t o[16];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            // dequant_pair gives (k, k + 4) pairs; the operand wants the eight inputs of a word in order.
+            const uint32_t word = words[half * 4 + w];
+            const uint32_t p0 = dequant_pair(word, zero2, scale2);
+            const uint32_t p1 = dequant_pair(word >> 4, zero2, scale2);
+            const uint32_t p2 = dequant_pair(word >> 8, zero2, scale2);
+            const uint32_t p3 = dequant_pair(word >> 12, zero2, scale2);
+            o[4 * w] = __byte_perm(p0, p1, 0x5410);
+            o[4 * w + 1] = __byte_perm(p2, p3, 0x5410);
+            o[4 * w + 2] = __byte_perm(p0, p1, 0x7632);
+            o[4 * w + 3] = __byte_perm(p2, p3, 0x7632);
+          }
+          if (kTensorOperands) {
+            tmem_store16(operand + half * 16, o);
+          } else {
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+              *reinterpret_cast<uint4*>(operand_row + (((half * 4 + w) ^ (row & 7)) << 4)) =
+                  make_uint4(o[4 * w], o[4 * w + 1], o[4 * w + 2], o[4 * w + 3]);
+          }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (kTensorOperands) {
+          tmem_stored();
+          tcgen05_fence_before();
+        } else {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
         __syncwarp();
         if (lane == 0) {
           mbarrier_arrive(&sh->ready[ready_slot]);
