@@ -208,7 +208,11 @@ __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_ker
     new_hi = fmaxf(new_hi, __shfl_xor_sync(0xffffffffu, new_hi, 2));
     // One warp, whose lanes all have their scores here (the maxima come of them): K's buffer takes the next tile's V. Also
     // where this tile's wait ran out: that V belongs to the next tile's barrier, which its K has armed.
-    if (kBuffers == 3 && threadIdx.x == 0) request_values(tile + 1, keys);
+    if (kBuffers == 3) {
+      __syncwarp();
+      if (threadIdx.x == 0) request_values(tile + 1, keys);
+      __syncwarp();  // the instructions below are those of a whole warp
+    }
     // A row with nothing visible yet keeps m = -inf; use 0 as the exponent base so that the power is 0.
     const float top_lo = new_lo == -INFINITY ? 0.0f : new_lo, top_hi = new_hi == -INFINITY ? 0.0f : new_hi;
     const float base_lo = top_lo * exponent_scale, base_hi = top_hi * exponent_scale;

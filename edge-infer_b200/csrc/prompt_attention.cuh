@@ -54,6 +54,7 @@ struct PaShared {
 
 // 16 columns of the warp's 32 lanes, without waiting for them.
 __device__ __forceinline__ void tmem_request16(uint32_t address, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
       "[%16];"
@@ -64,6 +65,7 @@ __device__ __forceinline__ void tmem_request16(uint32_t address, uint32_t (&r)[1
 }
 // Waits for the loads requested; the registers pass through so that nothing reads them earlier.
 __device__ __forceinline__ void tmem_loaded(uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
                  "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");

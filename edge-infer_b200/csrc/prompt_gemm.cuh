@@ -110,8 +110,11 @@ __device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint32_t desc_a, u
       : "r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(desc_high), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The loads, stores and waits of tensor memory are instructions of a whole warp that has not parted: each helper brings the
+// warp together first, since the code ahead of it may have lanes that store, arrive or take one more trip than others.
 __device__ __forceinline__ void tmem_load16(uint32_t address, float (&v)[16]) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
       "[%16];"
@@ -138,16 +141,21 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
 }
 
 __device__ __forceinline__ void tmem_store16(uint32_t address, const uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::
           "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
       "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(address)
       : "memory");
 }
-__device__ __forceinline__ void tmem_stored() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_stored() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 
 __device__ __forceinline__ void tmem_load8(uint32_t address, float (&v)[8]) {
   uint32_t r[8];
+  __syncwarp();
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(address)
@@ -584,6 +592,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
                                 pack_bf16(v[4] + bias, v[5] + bias), pack_bf16(v[6] + bias, v[7] + bias));
         }
       }
+      __syncwarp();  // as for tensor memory
       asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 2) * 2 + (warp & 1)) : "memory");
       if (complete) {
 #pragma unroll 1
