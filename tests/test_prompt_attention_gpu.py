@@ -109,3 +109,63 @@ def test_latent_attention_with_two_query_tiles(cuda, package):
     want = gikepel.GikepelOracle(c, weights).forward(ids)
     session = model.new_session(460)
     check_gikepel(layered_cases.run_portions(session, ids, [300, 150]), want, "bf16")
+
+
+def test_a_weight_that_dominates_is_not_rounded(cuda, package):
+    """One token of the first tile of 64, then one of the second that outweighs it by 2^n (1 + 0.9 2^-8): rounded to BF16 and
+    summed unrounded, that weight would take 0.9 2^-8 off the row; as the largest weight it is 1. All other tokens' weights
+    vanish. Every projection only selects, so the second layer's values are the first layer's attention output after two
+    roundings to BF16 (2^-8 / sqrt(3) RMS at most, each), whose mean over the 128 values of a head, weighted with their
+    squares, has a standard deviation of 2^-8 sqrt(2/3) sqrt(3/128) at most: 4.9e-4. The limit of 1.9e-3 is four times that;
+    the rounded weight's errors start at 0.75 x 3.5e-3 (a fifth of the row is the other token, a twentieth goes into the norm)."""
+    syn = package.synthetic
+    heads, hidden, history, rows, theta = 8, 2048, 128, 64, 1e7
+    half = hidden // 2
+    shape = package.Shape(vocab_size=512, n_layers=2, n_heads=heads, n_kv_heads=heads, hidden_size=hidden, intermediate_size=256,
+                          qk_norm=False, rope_theta=theta, max_position_embeddings=512)
+    tensors = syn.make_model(shape, seed=6)
+
+    def put(name, array):
+        tensors[name] = [(syn.DENSE, syn.float_to_bf16(array.astype(np.float32)))]
+
+    embedding = np.zeros((512, hidden))
+    embedding[:, :half] = 4.0           # the norm's size; the other half receives the attention's output
+    put("token_embeddings.weight", embedding)
+    normed = float(syn.bf16_to_float(syn.float_to_bf16(np.array([4 / np.sqrt(8 + 1e-6)], dtype=np.float32)))[0])
+    wq = np.zeros((heads, 128, hidden))
+    # Three values of a query that rotate by next to nothing (pairs of theta^-0.95 and less a token): coarse, fine, finest.
+    wq[:, 63, 0], wq[:, 62, 0], wq[:, 61, 0] = 16.0, 1.0, 2.0 ** -8
+    zeros = np.zeros((heads * 128, hidden))
+    for layer in range(2):
+        put(f"wq{layer}", wq.reshape(heads * 128, hidden))
+        put(f"wk{layer}", zeros)
+        put(f"wv{layer}", np.concatenate([zeros[:, :half], np.eye(half)], 1))
+        put(f"wo{layer}", np.concatenate([np.zeros((half, half)), np.eye(half)], 0))
+        put(f"w_gate{layer}", np.zeros((256, hidden)))
+        put(f"w_down{layer}", np.zeros((hidden, 256)))
+    model = package.Model(shape, tensors)
+
+    def bf16(x):
+        return syn.bf16_to_float(syn.float_to_bf16(np.asarray(x, dtype=np.float32))).astype(np.float64)
+
+    unit = normed / np.sqrt(128.0) * np.log2(np.e)     # exponents of two per unit of key value 62
+    k, v = np.zeros((history, heads, 128)), np.zeros((history, heads, 128))
+    first, second = 10, 100
+    k[[first, second], :, 63] = 30.0                   # 86 powers of two above the other tokens
+    n = 2 + np.arange(heads) % 6
+    wanted = (n + np.log2(1 + 0.9 * 2.0 ** -8)) / unit
+    k[second, :, 62] = bf16(wanted)
+    k[second, :, 61] = bf16((wanted - k[second, :, 62]) * 2.0 ** 8)
+    gap = 2.0 ** ((k[second, :, 62] + k[second, :, 61] * 2.0 ** -8) * unit)
+    v[[first, second]] = bf16(np.random.default_rng(7).standard_normal((2, heads, 128)))
+    expected = (v[first] + gap[:, None] * v[second]) / (1 + gap[:, None])
+
+    session = model.new_session(256)
+    session.prefill([1] * history)
+    flat = [syn.float_to_bf16(x.reshape(history, heads * 128).astype(np.float32)) for x in (k, v)]
+    session.write_kv(0, 0, *flat)
+    session.extend([1] * rows)
+    got = syn.bf16_to_float(session.read_kv(1)[1])[history:].reshape(rows, heads, 128).astype(np.float64)
+    got *= np.sqrt((16 * half + (expected ** 2).sum()) / hidden + 1e-6)
+    share = (got * expected).sum(-1) / (expected ** 2).sum(-1)
+    assert np.abs(share - 1).max() <= 1.9e-3, np.abs(share - 1).max(0)
