@@ -87,10 +87,10 @@ class PromptShapes {
  public:
   // int4 takes one feature tile: two of them dequantise the weights of 256 features per K block, which at 128-240 columns
   // took 1500-1900 cycles where one tile with as many accumulator columns takes 1226.
-  // `gated`: a block computes gate and up features side by side; BF16 takes a feature tile of each, int4 half a tile of each.
+  // `gated`: a block computes gate and up features side by side, half a tile of each or, where it takes two tiles, one of each.
   PromptShapes(bool awq, int rows, int N, int K, int multiprocessors, bool gated = false)
-      : awq_(awq), rows_(rows), n_(N), k_(K), multiprocessors_(multiprocessors) {
-    for (int feature_tiles = gated && !awq ? 2 : 1; feature_tiles <= (awq ? 1 : 2); ++feature_tiles)
+      : awq_(awq), gated_(gated), rows_(rows), n_(N), k_(K), multiprocessors_(multiprocessors) {
+    for (int feature_tiles = 1; feature_tiles <= (awq ? 1 : 2); ++feature_tiles)
       for (int token_tiles = 1; token_tiles <= 2; ++token_tiles) {
         const int most = std::min(kPromptMaxColumns, kPromptTmemColumns / (feature_tiles * token_tiles) / 16 * 16);
         const int fewest = (rows + most * token_tiles - 1) / (most * token_tiles);
@@ -113,9 +113,13 @@ class PromptShapes {
     for (int i = 0; i < count_; ++i) {
       const Shape& s = shapes_[i];
       const long long waves = (s.blocks * ksplit + multiprocessors_ - 1) / multiprocessors_;
-      double cycles = std::max(2500.0 + waves * (k_blocks * s.block + s.fixed), s.memory) + more;
+      double cycles = 2500.0 + waves * (k_blocks * s.block + s.fixed);
+      const bool pair = gated_ && s.tile.feature_tiles == 2;
+      if (pair) cycles *= kPairedTiles;
+      cycles = std::max(cycles, s.memory) + more;
       if (s.tile.x_stages < 3) cycles *= 1.25;  // two stages do not hide a copy's latency
-      if (!result.tile.columns || cycles < result.cycles) result = PromptChoice{s.tile, cycles};
+      const bool better = cycles < result.cycles || (pair && cycles == result.cycles && result.tile.feature_tiles == 1);
+      if (!result.tile.columns || better) result = PromptChoice{s.tile, cycles};
     }
     return result;
   }
@@ -181,7 +185,16 @@ class PromptShapes {
     return cycles;
   }
 
-  bool awq_;
+  // BF16 gate and up rows in a feature tile each are charged this share of the estimate against half a tile each, whose warps
+  // have to exchange their values (half the units a block, so twice the blocks), and they win where both wait for HBM. Fitted
+  // between the sizes where one or the other is faster; a layer of a prompt, whole tiles -> half tiles, us: 6144 x 1024 at 33
+  // rows 39.2 -> 38.2, at 256 49.2 -> 47.7, but at 700 65.8 -> 68.6 (*); 12288 x 2048 at 40 rows 53.0 -> 49.6, at 128 59.9 ->
+  // 57.4, but at 200 66.0 -> 70.0 (*); 37888 x 3584 at 320 rows, where whole tiles take two groups of tokens and fetch the
+  // weights twice, 220 -> 195, but at 33 112 -> 118.6 (*). (*: with one kernel for both, about 1 us slower.) Over those, 17920 x 1536, 19456 x 2560 and 24576 x 4096 at 33 to 2040 rows the projection
+  // and units chosen here take 1 to 10 % off a layer with a kernel of its own for the units, and are slower nowhere.
+  static constexpr double kPairedTiles = 0.85;
+
+  bool awq_, gated_;
   int rows_, n_, k_, multiprocessors_, count_ = 0;
   Shape shapes_[16];
 };

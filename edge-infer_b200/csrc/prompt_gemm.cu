@@ -28,9 +28,10 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device != device) {
     EI_CUDA(cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device));
-    for (const auto kernel : {prompt_gemm_kernel<true, false, false>, prompt_gemm_kernel<true, false, true>,
-                              prompt_gemm_kernel<true, true, false>, prompt_gemm_kernel<true, true, true>,
-                              prompt_gemm_kernel<false, false, false>, prompt_gemm_kernel<false, true, false>})
+    for (const auto kernel : {prompt_gemm_kernel<true, kUngated, false>, prompt_gemm_kernel<true, kUngated, true>,
+                              prompt_gemm_kernel<true, kHalfTiles, false>, prompt_gemm_kernel<true, kHalfTiles, true>,
+                              prompt_gemm_kernel<false, kUngated, false>, prompt_gemm_kernel<false, kHalfTiles, false>,
+                              prompt_gemm_kernel<false, kWholeTiles, false>})
       EI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPromptSharedLimit)));
     configured_device = device;
   }
@@ -45,6 +46,8 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   q.ksplit = ksplit;
   q.prompt = PromptShapes(awq, p.M, p.N, p.K, multiprocessors, gated).best(ksplit, p.epilogue == kEpiPartial, false).tile;
   if (awq) q.prompt = prompt_tensor_operands(q.prompt);
+  const bool halves = gated && q.prompt.feature_tiles == 1;  // gate and up rows share a tile and come as a box each
+  const cuuint32_t rows_of_box = halves ? kPromptFeatures / 2 : kPromptFeatures;
   PromptMaps maps{};
   {
     const cuuint64_t dims[2] = {cuuint64_t(p.K), cuuint64_t(p.M)};
@@ -57,14 +60,14 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
     if (!aligned_16(p.qweight) || (p.K / 8) % 4) throw std::invalid_argument("prompt GEMM: packed weight rows must be 16-byte aligned");
     const cuuint64_t dims[2] = {cuuint64_t(p.K / 8), cuuint64_t(p.N)};
     const cuuint64_t strides[1] = {cuuint64_t(p.K / 8) * 4};
-    const cuuint32_t box[2] = {kPromptBlockK / 8, cuuint32_t(gated ? kPromptFeatures / 2 : kPromptFeatures)};
+    const cuuint32_t box[2] = {kPromptBlockK / 8, rows_of_box};
     encode_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, p.qweight, dims, strides, box,
                CU_TENSOR_MAP_SWIZZLE_NONE, "prompt int4 weights");
   } else {
     if (!aligned_16(p.w) || p.ldw % 8) throw std::invalid_argument("prompt GEMM: weight rows must be 16-byte aligned");
     const cuuint64_t dims[2] = {cuuint64_t(p.K), cuuint64_t(p.N)};
     const cuuint64_t strides[1] = {cuuint64_t(p.ldw) * 2};
-    const cuuint32_t box[2] = {kPromptBlockK, kPromptFeatures};
+    const cuuint32_t box[2] = {kPromptBlockK, rows_of_box};
     encode_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.w, dims, strides, box,
                CU_TENSOR_MAP_SWIZZLE_128B, "prompt weights");
   }
@@ -72,9 +75,11 @@ void launch_prompt_gemm(bool awq, const GemmParams& p, cudaStream_t stream, bool
   const size_t shared = size_t(prompt_ring_bytes(q.prompt)) + kPromptSharedExtra;
   const dim3 grid((p.N + features - 1) / features, (p.M + tokens - 1) / tokens, ksplit);
   const bool tensor = q.prompt.tensor_operands;
-  const auto kernel = !awq    ? (gated ? prompt_gemm_kernel<false, true, false> : prompt_gemm_kernel<false, false, false>)
-                      : gated ? (tensor ? prompt_gemm_kernel<true, true, true> : prompt_gemm_kernel<true, true, false>)
-                              : (tensor ? prompt_gemm_kernel<true, false, true> : prompt_gemm_kernel<true, false, false>);
+  const auto kernel = !awq    ? (halves ? prompt_gemm_kernel<false, kHalfTiles, false>
+                                 : gated ? prompt_gemm_kernel<false, kWholeTiles, false>
+                                         : prompt_gemm_kernel<false, kUngated, false>)
+                      : gated ? (tensor ? prompt_gemm_kernel<true, kHalfTiles, true> : prompt_gemm_kernel<true, kHalfTiles, false>)
+                              : (tensor ? prompt_gemm_kernel<true, kUngated, true> : prompt_gemm_kernel<true, kUngated, false>);
   launch(kernel, grid, dim3(kPromptThreads), shared, stream, pdl, maps, q);
 }
 

@@ -270,7 +270,11 @@ __device__ __forceinline__ void gated_units(int glu, float limit, uint32_t (&gat
   }
 }
 
-template <bool kAwq, bool kGated, bool kTensorOperands>
+// Where a block has its gate and up rows: in the halves of its one feature tile, or (BF16) in a tile each. Instances of their own:
+// one kernel that asked at run time took 1 us of 38 more a layer at 33 rows of 6144 x 1024.
+enum PromptGate { kUngated, kHalfTiles, kWholeTiles };
+
+template <bool kAwq, int kGate, bool kTensorOperands>
 __global__ void __launch_bounds__(kPromptThreads, 1)
     prompt_gemm_kernel(const __grid_constant__ PromptMaps maps, const GemmParams p) {
   extern __shared__ unsigned char prompt_smem_raw[];
@@ -280,7 +284,8 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
   PromptShared* sh = reinterpret_cast<PromptShared*>(smem + prompt_ring_bytes(p.prompt));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // kGated: the block's rows are n0 ... of the gate and, from `pairs` on, as many of the up projection; the epilogue leaves
-  // their gated units. BF16: tile 0 is gate, tile 1 up; int4: the one tile's first and second half are.
+  // their gated units. The one feature tile's first and second half are gate and up, or (BF16) the first and second tile.
+  constexpr bool kGated = kGate != kUngated;
   const int pairs = p.N / 2;
   const int n0 = blockIdx.x * (kPromptFeatures * p.prompt.feature_tiles / (kGated ? 2 : 1)), t0 = blockIdx.y * block_tokens;
   const int feature_tiles =
@@ -337,8 +342,10 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
             tma_load_2d(to, &maps.weights, word, n0 + f * kPromptFeatures, &full[s]);
             if (kGated) tma_load_2d(to + kPromptRawBytes / 2, &maps.weights, word, pairs + n0, &full[s]);
           } else {
-            tma_load_2d(w_ring + s * w_bytes + f * kPromptWeightBytes, &maps.weights, (kb_begin + kb) * kPromptBlockK,
-                        n0 + (kGated ? f * pairs : f * kPromptFeatures), &full[s]);
+            unsigned char* const to = w_ring + s * w_bytes + f * kPromptWeightBytes;
+            const int input = (kb_begin + kb) * kPromptBlockK;
+            tma_load_2d(to, &maps.weights, input, n0 + (kGated ? f * pairs : f * kPromptFeatures), &full[s]);
+            if (kGate == kHalfTiles) tma_load_2d(to + kPromptWeightBytes / 2, &maps.weights, input, pairs + n0, &full[s]);
           }
         }
       } else {
@@ -544,17 +551,17 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
       }
     };
     // The same for pairs of two tokens' values.
-    const uint32_t halves = odd ? 0x3276u : 0x5410u;
+    const uint32_t own_halves = odd ? 0x3276u : 0x5410u;
     auto store_words = [&](const auto& words, int token, int first_unit) {
 #pragma unroll
       for (int i = 0; i < int(sizeof(words) / sizeof(uint32_t)); ++i) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, words[i], 1);
         const int mine = token + 2 * i + (odd ? 1 : 0);
         if (mine < p.M && first_unit < pairs)
-          *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_unit) = __byte_perm(words[i], other, halves);
+          *reinterpret_cast<uint32_t*>(p.out + size_t(mine) * p.out_stride + first_unit) = __byte_perm(words[i], other, own_halves);
       }
     };
-    if (kGated && !kAwq && complete) {
+    if (kGate == kWholeTiles && complete) {
       // A lane has a unit's gate in one accumulator and its up value in the other.
       const int unit = n0 + quarter * 32 + lane;
       const float gate_bias = p.bias && unit < pairs ? __bfloat162float(p.bias[unit]) : 0.0f;
@@ -573,7 +580,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1)
         gated_units(p.glu, p.glu_limit, gates, ups);
         store_words(gates, t0 + c, unit & ~1);
       }
-    } else if (kGated && kAwq) {
+    } else if (kGate == kHalfTiles) {
       // A unit's gate is in lane l of the first two quarters, its up value in the same lane two quarters on: the two warps
       // hand one another half the tokens of each group of 16 through the rings, which nothing uses any more, and each
       // finishes the other half.
