@@ -235,9 +235,8 @@ __device__ __forceinline__ void prompt_drain(PromptShared* sh, const PromptTile&
 // The gated units of kWords pairs of gate and up values, which replace the gates. Values travel as BF16 pairs, which take half
 // the conversions of single ones: the epilogue of 128 x 416 sums is bound by its instructions (two of which per unit are
 // those of the exponential and the reciprocal). The SiLU's branches for tiny and very negative gates are taken only where one
-// of the values needs them; elsewhere 1 + e^-x is far from where the fast quotient would have to scale. The gates of tokens and
-// units that do not exist (from value `live` on) are zeros, which would take all lanes into those branches (0.4 to 0.5 us of a
-// layer at 33 or 56 rows of 24576 x 4096 and 257 or 333 of 12288 x 2048).
+// of the values needs them. The gates of tokens and units that do not exist (from value `live` on) are zeros, which would take
+// all lanes into those branches (0.4 to 0.5 us of a layer at 33 or 56 rows of 24576 x 4096 and 257 or 333 of 12288 x 2048).
 template <int kWords>
 __device__ __forceinline__ void gated_units(int glu, float limit, int live, uint32_t (&gate)[kWords], const uint32_t (&up)[kWords]) {
   if (live <= 0) return;
@@ -268,11 +267,7 @@ __device__ __forceinline__ void gated_units(int glu, float limit, int live, uint
   } else {
 #pragma unroll
     for (int i = 0; i < kWords; ++i) {
-      auto silu = [](float x) {
-        float r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-x)));
-        return x * r;
-      };
+      auto silu = [](float x) { return __fdividef(x, 1.0f + __expf(-x)); };  // silu_value's main branch
       const uint32_t a = pack_bf16(silu(bf16_lo(gate[i])), silu(bf16_hi(gate[i])));
       const uint32_t signs = a ^ up[i];  // a zero of the product's sign, as in multiply_activated
       gate[i] = pack_bf16(__fmaf_ieee_rn(bf16_lo(a), bf16_lo(up[i]), __uint_as_float((signs << 16) & 0x80000000u)),

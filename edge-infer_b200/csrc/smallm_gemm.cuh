@@ -105,11 +105,6 @@ __device__ __forceinline__ float multiply_activated(float activated, float up) {
 __device__ __forceinline__ float silu_multiply_value(float gate, float up) {
   return multiply_activated(round_bf16(silu_value(gate)), up);
 }
-// The same for a gate that is not rare.
-__device__ __forceinline__ float silu_multiply_common(float gate, float up) {
-  return multiply_activated(round_bf16(__fdividef(gate, 1.0f + __expf(-gate))), up);
-}
-
 __device__ __forceinline__ float clamped_glu_value(float gate, float up, float limit) {
   const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
   return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
