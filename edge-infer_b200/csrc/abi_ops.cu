@@ -516,6 +516,7 @@ static void run_attention(const ei_context* ctx, ei_view3 q, ei_view3 k, ei_view
   p.host_offset = int(offset);
   p.chunk = attention_chunk_for(length);
   p.max_splits = int((length + p.chunk - 1) / p.chunk);
+  if (!device_offset) p.live_blocks = p.max_splits * p.kv_heads;
   p.scratch = static_cast<float*>(scratch);
   p.out = static_cast<bf16*>(out.data);
   p.out_stride = int(out.stride[0]);

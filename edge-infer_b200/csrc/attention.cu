@@ -5,7 +5,7 @@
 // one chunk of the sequence, and serves every query row of every query head of that KV group
 // (rows * heads/kv_heads <= 112 stacked rows, one 16-row MMA tile per warp). K and V tiles of
 // 64 tokens are brought into shared memory by TMA (one tiled copy each for K and V, issued by one thread,
-// completing on an mbarrier; a ring of three tiles per block, every wait bounded) in the 128-byte-swizzled
+// completing on an mbarrier; a ring of up to three tiles per block, every wait bounded) in the 128-byte-swizzled
 // layout [half of the head][token][128 B], which makes the fragment loads conflict-free. Scores, running maxima and sums
 // stay in FP32; numerators are rounded to BF16 only as the A operand of the PV product while the
 // denominator adds the unrounded values - the staging of the reference kernel
@@ -13,6 +13,7 @@
 // caller scratch and a second kernel merges the live chunks in FP32 and rounds once.
 // The position of the first query row is read from device memory, so a captured graph can be
 // replayed while the context grows; blocks beyond the live length return immediately.
+#include "attention_ring.hpp"
 #include "kernels.cuh"
 #include "prompt_attention.cuh"
 
@@ -28,17 +29,12 @@ constexpr int kDim = 128;
 constexpr int kPartial = 132;      // floats per (split, row, head): 128 outputs, m, l, padding
 constexpr int kTileBytes = kTile * kDim * 2;
 
-// The ring: K and V tiles in turn, a buffer each. A block of several warps has four buffers, two tiles; two such blocks share an
-// SM (registers). A block of one warp knows without a barrier that K has been read, hands K's buffer on as soon as the scores
-// stand and gets by on three, so that four blocks share an SM. What bounds those is the chain of one warp, 2 us a tile, at two
-// blocks on an SM (rings of three tiles, 97 KB) 0.66 of the HBM peak: 64 splits of 8 KV heads were two waves, now they are one.
-// Steps, three tiles a block -> this: 8B int4, 4 rows behind 30 000 tokens 2.92 -> 2.72 ms, 9 rows behind 2000 2.583 -> 2.566,
-// 64 x 5 rows of 7B int4 9.34 -> 9.24; 1.7B and 0.6B the same. (Two tiles, so that three one-warp blocks share an SM: 3.03 at
-// the first size, where 28 of 472 blocks make a second wave that costs almost as much as the first.)
+// The ring: K and V tiles in turn, a buffer each; how many is attention_ring.hpp's choice. A block of one warp knows without a
+// barrier that K has been read: with three buffers it hands K's on as soon as the scores stand.
 constexpr size_t attention_shared(int buffers) { return size_t(buffers) * kTileBytes + 1024 /* alignment */ + 64; }
 
 struct AttentionShared {
-  uint64_t full[2];  // by tile, of either parity
+  uint64_t full[3];  // of the tiles under way
   int failed;
 };
 
@@ -52,6 +48,7 @@ __device__ __forceinline__ int tile_offset(int token, int chunk) {
 // merge kernel.
 template <int kBuffers>
 __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_kernel(const __grid_constant__ AttentionParams p) {
+  constexpr int kTiles = kBuffers == 6 ? 3 : 2;  // under way
   extern __shared__ unsigned char attention_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(attention_smem_raw) + 1023) &
                                                          ~uintptr_t(1023));
@@ -90,7 +87,7 @@ __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_ker
   const int tiles = (end - start + kTile - 1) / kTile;
 
   if (threadIdx.x == 0) {
-    for (int b = 0; b < 2; ++b) mbarrier_init(&sh->full[b], 1);
+    for (int b = 0; b < kTiles; ++b) mbarrier_init(&sh->full[b], 1);
     sh->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -98,21 +95,22 @@ __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_ker
   // One thread requests the boxes of 64 tokens of this KV head. K's arms the tile's barrier for both.
   auto request_keys = [&](int tile, int buffer) {
     if (tile >= tiles) return;
-    mbarrier_expect_tx(&sh->full[tile & 1], uint32_t(2 * kTileBytes) + (tile == 0 ? p.fault_tx : 0u));
-    tma_load_5d(smem + buffer * kTileBytes, k_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile & 1]);
+    mbarrier_expect_tx(&sh->full[tile % kTiles], uint32_t(2 * kTileBytes) + (tile == 0 ? p.fault_tx : 0u));
+    tma_load_5d(smem + buffer * kTileBytes, k_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile % kTiles]);
   };
   auto request_values = [&](int tile, int buffer) {
     if (tile >= tiles) return;
-    tma_load_5d(smem + buffer * kTileBytes, v_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile & 1]);
+    tma_load_5d(smem + buffer * kTileBytes, v_map, 0, start + tile * kTile, 0, kv_head, layer, &sh->full[tile % kTiles]);
   };
 
   const bool settled = end <= offset;  // no row of this chunk is written by the preceding kernel
   if (!settled) grid_dependency_wait();
   if (threadIdx.x == 0) {
-    request_keys(0, 0);
-    request_values(0, 1);
-    request_keys(1, 2);
-    if (kBuffers == 4) request_values(1, 3);
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) {
+      request_keys(t, 2 * t);
+      if (2 * t + 1 < kBuffers) request_values(t, 2 * t + 1);
+    }
   }
   if (settled) grid_dependency_wait();  // the queries come from the preceding kernel
   // Only now: a kernel that triggers after its own wait lets its successor's prologue see everything up to the
@@ -149,7 +147,7 @@ __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_ker
   int tile = 0, keys = 0;  // the tile, the buffer of its K
   bool gave_up = false;
   for (; tile < tiles; ++tile) {
-    if (!mbarrier_wait(&sh->full[tile & 1], (tile >> 1) & 1, wait_limit)) sh->failed = 1;
+    if (!mbarrier_wait(&sh->full[tile % kTiles], (tile / kTiles) & 1, wait_limit)) sh->failed = 1;
     const int values = keys + 1 == kBuffers ? 0 : keys + 1;
     unsigned char* ks = smem + keys * kTileBytes;
     unsigned char* vs = smem + values * kTileBytes;
@@ -263,17 +261,17 @@ __global__ void __launch_bounds__(kBuffers == 3 ? 32 : 224) verify_attention_ker
     gave_up = sh->failed != 0;  // written before the barrier by any thread whose wait ran out: block-uniform
     if (gave_up) break;
     if (threadIdx.x == 0) {
-      request_keys(tile + 2, kBuffers == 4 ? keys : values);
-      if (kBuffers == 4) request_values(tile + 2, values);
+      request_keys(tile + kTiles, kBuffers == 3 ? values : keys);
+      if (kBuffers != 3) request_values(tile + kTiles, values);
     }
-    keys = keys >= 2 ? keys + 2 - kBuffers : keys + 2 == kBuffers ? 0 : 2;
+    keys = keys + 2 < kBuffers ? keys + 2 : keys + 2 - kBuffers;
   }
   if (gave_up) {
     // Copies still in flight write into this block's shared memory: wait for them (bounded) before leaving. The
     // copy of tile 0 carries the test hook's unmet expectation when that is armed and is known not to complete.
     if (threadIdx.x == 0) {
-      for (int t = max(tile, p.fault_tx ? 1 : 0); t < min(tile + 2, tiles); ++t)
-        mbarrier_wait(&sh->full[t & 1], (t >> 1) & 1, wait_limit);
+      for (int t = max(tile, p.fault_tx ? 1 : 0); t < min(tile + kTiles, tiles); ++t)
+        mbarrier_wait(&sh->full[t % kTiles], (t / kTiles) & 1, wait_limit);
       if (p.status) atomicOr(p.status, 4);
     }
     return;
@@ -498,13 +496,17 @@ size_t attention_scratch_bytes(size_t rows, size_t heads, size_t kv_length) {
 }
 
 namespace {
+auto verify_attention(int buffers) {
+  return buffers == 3 ? verify_attention_kernel<3> : buffers == 4 ? verify_attention_kernel<4> : verify_attention_kernel<6>;
+}
+
 void configure_attention_kernels() {
   static thread_local int configured_device = -1;
   int device = 0;
   EI_CUDA(cudaGetDevice(&device));
   if (configured_device == device) return;
-  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attention_shared(3))));
-  EI_CUDA(cudaFuncSetAttribute(verify_attention_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attention_shared(4))));
+  for (const int buffers : {3, 4, 6})
+    EI_CUDA(cudaFuncSetAttribute(verify_attention(buffers), cudaFuncAttributeMaxDynamicSharedMemorySize, int(attention_shared(buffers))));
   EI_CUDA(cudaFuncSetAttribute(prompt_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PaLayout<kDim>::kTotal)));
   configured_device = device;
 }
@@ -540,10 +542,8 @@ void launch_verify_attention(const AttentionParams& p, cudaStream_t stream, bool
   configure_attention_kernels();
   const AttentionParams q = with_maps(p);
   const unsigned sessions = q.slots ? unsigned(q.sessions) : 1u;
-  // One warp: three buffers, four blocks on an SM; more: registers allow two blocks, which may as well hold two tiles.
-  const int buffers = warps == 1 ? 3 : 4;
-  launch(warps == 1 ? verify_attention_kernel<3> : verify_attention_kernel<4>, dim3(q.kv_heads, q.max_splits, sessions),
-         dim3(warps * 32), attention_shared(buffers), stream, pdl, q);
+  const int buffers = attention_buffers(warps, q.live_blocks, q.chunk / kTile, device_multiprocessors());
+  launch(verify_attention(buffers), dim3(q.kv_heads, q.max_splits, sessions), dim3(warps * 32), attention_shared(buffers), stream, pdl, q);
   if (q.slots && !q.merge_blocks)
     launch(attention_merge_wide_kernel, dim3((q.rows * q.heads * q.sessions + 3) / 4), dim3(128), 0, stream, pdl, q);
   else

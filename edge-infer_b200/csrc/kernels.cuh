@@ -146,6 +146,7 @@ struct AttentionParams {
   int host_offset;
   int chunk;                // tokens per split (multiple of 64)
   int max_splits;
+  int live_blocks;          // blocks of the grid that will have tokens, or somewhat more; 0: not known
   float* scratch;           // [max_splits][rows * heads][132]
   bf16* out;                // row r, head h at out + r * out_stride + h * 128
   int out_stride;

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <limits>
 
+#include "attention_ring.hpp"
 #include "layered.cuh"
 
 namespace ei {
@@ -360,7 +361,7 @@ void enqueue_commit(ei_session& s, int rows, bool folded) {
 // and acceptance stay per session. The first session lends its workspace and stream.
 struct ei_batch {
   std::vector<ei_session*> sessions;
-  cudaGraphExec_t graphs[kMaxRows + 1] = {};  // by rows per session
+  cudaGraphExec_t graphs[3][kMaxRows + 1] = {};  // by the attention's ring and rows per session
   // Wide form (more than 16 stacked rows): the sessions' slots on the device, and buffers sized on first use
   // for sessions * rows stacked rows.
   SessionSlot* slots = nullptr;
@@ -642,6 +643,18 @@ void enqueue_prompt_segment(ei_session& s, int rows, bool head) {
   enqueue_commit(s, rows, true);
 }
 
+// Attention blocks of the next step that have tokens, by the longest the history can be.
+int live_attention_blocks(const ei_session& s, int rows, int chunk) {
+  const size_t length = std::min(s.capacity, std::max(s.context, s.bound) + size_t(rows));
+  return int(s.model->config.n_kv_heads * ((length + chunk - 1) / chunk));
+}
+// Which of a step's graphs has the ring that its attention takes.
+int attention_ring(const ei_model& m, int rows, int chunk, int live_blocks) {
+  const int warps = (rows * int(m.config.n_heads / m.config.n_kv_heads) + 15) / 16;
+  const int buffers = attention_buffers(warps, live_blocks, chunk / 64, m.multiprocessors);
+  return buffers == 3 ? 0 : buffers == 4 ? 1 : 2;
+}
+
 // Enqueues one forward of `rows` tokens at the device-side context length.
 void enqueue_step(ei_session& s, int rows, StepKind kind, bf16* logits_out) {
   if (s.model->layered) {
@@ -710,6 +723,7 @@ void enqueue_step(ei_session& s, int rows, StepKind kind, bf16* logits_out) {
     a.status = &s.control->status;
     a.chunk = s.attention_chunk;
     a.max_splits = s.attention_splits;
+    a.live_blocks = live_attention_blocks(s, rows, s.attention_chunk);
     a.scratch = s.attention_scratch;
     a.out = s.attention;
     a.out_stride = heads * 128;
@@ -772,7 +786,9 @@ void submit_step(ei_session& s, int rows, StepKind kind) {
     enqueue_step(s, rows, kind, nullptr);
     return;
   }
-  cudaGraphExec_t& exec = s.graphs[int(kind)][rows];
+  const int ring =
+      s.model->layered ? 0 : attention_ring(*s.model, rows, s.attention_chunk, live_attention_blocks(s, rows, s.attention_chunk));
+  cudaGraphExec_t& exec = s.graphs[int(kind)][ring][rows];
   if (!exec) {
     // Warm run outside capture: sets kernel attributes, loads modules, and does real work.
     enqueue_step(s, rows, kind, nullptr);
@@ -798,6 +814,12 @@ void submit_step(ei_session& s, int rows, StepKind kind) {
   }
   tick(s);
   EI_CUDA(cudaGraphLaunch(exec, s.stream));
+}
+
+int live_attention_blocks(const ei_batch& batch, int rows, int chunk) {
+  int blocks = 0;
+  for (const ei_session* s : batch.sessions) blocks += live_attention_blocks(*s, rows, chunk);
+  return blocks;
 }
 
 // One verify step of every session of the batch, `rows` tokens each, on the leader's stream and workspace.
@@ -860,6 +882,7 @@ void enqueue_batch_step(ei_batch& batch, int rows) {
     a.kv_heads = kv_heads;
     a.chunk = lead.attention_chunk;
     a.max_splits = lead.attention_splits;
+    a.live_blocks = live_attention_blocks(batch, rows, a.chunk);
     a.scratch = lead.attention_scratch;
     a.scratch_stride = scratch_floats;
     a.out = lead.attention;
@@ -1000,6 +1023,7 @@ void enqueue_wide_batch_step(ei_batch& batch, int rows) {
     // write and merge, the per-block set-up paid once per eight tiles), still at most 64 splits.
     a.chunk = std::max(512, lead.attention_chunk);
     a.max_splits = int((lead.capacity + a.chunk - 1) / a.chunk);
+    a.live_blocks = live_attention_blocks(batch, rows, a.chunk);
     a.scratch = batch.attention_scratch;
     a.scratch_stride = batch.scratch_stride;
     a.out = ws.attention;
@@ -1036,7 +1060,8 @@ void submit_batch_step(ei_batch& batch, int rows) {
     enqueue_batch_step(batch, rows);
     return;
   }
-  cudaGraphExec_t& exec = batch.graphs[rows];
+  const int ring = attention_ring(*lead.model, rows, lead.attention_chunk, live_attention_blocks(batch, rows, lead.attention_chunk));
+  cudaGraphExec_t& exec = batch.graphs[ring][rows];
   if (!exec) {
     enqueue_batch_step(batch, rows);  // warm run: real work, kernel attributes, first-use set-up
     cudaGraph_t graph = nullptr;
@@ -1302,8 +1327,9 @@ void ei_session_destroy(ei_session* s) {
   if (previous != s->model->device) cudaSetDevice(s->model->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
   for (auto& kind : s->graphs)
-    for (auto& exec : kind)
-      if (exec) cudaGraphExecDestroy(exec);
+    for (auto& ring : kind)
+      for (auto& exec : ring)
+        if (exec) cudaGraphExecDestroy(exec);
   if (s->host_tokens) cudaFreeHost(s->host_tokens);
   if (s->host_control) cudaFreeHost(s->host_control);
   if (s->arena) cudaFree(s->arena);
@@ -1606,8 +1632,9 @@ ei_status ei_batch_create(ei_session* const* sessions, size_t count, ei_batch** 
 
 void ei_batch_destroy(ei_batch* batch) {
   if (!batch) return;
-  for (auto& exec : batch->graphs)
-    if (exec) cudaGraphExecDestroy(exec);
+  for (auto& ring : batch->graphs)
+    for (auto& exec : ring)
+      if (exec) cudaGraphExecDestroy(exec);
   if (!batch->sessions.empty()) cudaStreamSynchronize(batch->sessions[0]->stream);
   if (batch->slots) cudaFree(batch->slots);
   if (batch->maps) cudaFree(batch->maps);

@@ -112,8 +112,9 @@ struct ei_session {
                                    // expectation it cannot meet, so that its bounded waits run out
   size_t launches = 0, launches_per_step[ei::kMaxRows + 1] = {};
   size_t prefill_target_row = 0;  // where in `targets` the last prefill left the greedy token of its last row
-  // graphs: [kind][rows]; kind 0 verify (host tokens), 1 verify (device drafts), 2 decode (commit all)
-  cudaGraphExec_t graphs[3][ei::kMaxRows + 1] = {};
+  // graphs: [kind][ring][rows]; kind 0 verify (host tokens), 1 verify (device drafts), 2 decode (commit all); ring: a form of the
+  // attention's (the results are the same bits)
+  cudaGraphExec_t graphs[3][3][ei::kMaxRows + 1] = {};
 };
 
 namespace ei {
