@@ -624,6 +624,11 @@ void enqueue_prompt_segment(ei_session& s, int rows, bool head) {
     a.status = &s.control->status;
     a.out = ws.attention;
     a.out_stride = heads * 128;
+    if (s.inject_attention_polls) {
+      a.wait_limit = s.inject_attention_polls;
+      a.fault_tx = 16;
+      s.inject_attention_polls = 0;  // one launch only
+    }
     tick(s);
     launch_prompt_attention(a, s.stream, pdl);
 

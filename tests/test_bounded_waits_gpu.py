@@ -64,3 +64,25 @@ def test_prompt_gemm_waits_once_for_what_is_in_flight(cuda, package, quant):
     assert taken < 2.5 * limit, (taken, limit)
     session.prefill(prompt)
     assert np.array_equal(session.read_logits(1), expected)
+
+
+@pytest.mark.parametrize("heads,kv_heads,rows", [(8, 8, 100), (40, 40, 300), (60, 20, 300)])
+def test_prompt_attention_gives_up_with_its_copies_in_flight(cuda, package, heads, kv_heads, rows):
+    """The first copy of keys of every block is told to bring 16 bytes more than it does. Blocks of one query tile; of two, whose
+    softmax warps take turns; of two whose queries are loaded instead of copied (groups of three). Afterwards the session and the
+    same prompt are as before."""
+    syn = package.synthetic
+    shape = package.Shape(vocab_size=512, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, hidden_size=256, intermediate_size=256,
+                          max_position_embeddings=512)
+    model = package.Model(shape, syn.make_model(shape, seed=7))
+    session = model.new_session(512)
+    prompt = syn.make_prompt(4, rows, shape.vocab_size)
+    session.prefill(prompt)
+    expected = session.read_logits(1).copy()
+    for _ in range(2):
+        session.inject_attention_wait_timeout(2000)
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            session.prefill(prompt)
+        session.prefill(prompt)
+        assert np.array_equal(session.read_logits(1), expected)
+    assert session.verify([7, 8]).emitted >= 1   # the hook was the prompt's, not the next step's
