@@ -58,9 +58,9 @@ def test_edges_of_tiles(cuda, package, heads, kv_heads, history, rows):
     assert_same_rows(syn, wide, narrow, history, len(ids))
 
 
-@pytest.mark.parametrize("heads,kv_heads,rows", [(40, 40, 300), (32, 8, 610), (32, 8, 600), (56, 8, 400)])
+@pytest.mark.parametrize("heads,kv_heads,rows", [(40, 40, 300), (32, 8, 610), (32, 8, 600), (56, 8, 400), (40, 40, 428)])
 def test_blocks_of_two_query_tiles(cuda, package, heads, kv_heads, rows):
-    """More blocks than half the multiprocessors; the last block's second query tile has 44, 8, 0 and 112 rows."""
+    """More blocks than half the multiprocessors; the last block's second query tile has 0, 8, 0, 112 and 44 rows."""
     syn = package.synthetic
     shape = two_layers(package, heads, kv_heads)
     model = package.Model(shape, syn.make_model(shape, seed=4, vary_norms=True))

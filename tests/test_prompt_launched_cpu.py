@@ -1,6 +1,6 @@
-"""The tiles that prompt projections with the gated unit are launched with (csrc/prompt_choice.hpp: the shape chosen and, for int4, where
-its operands stand): those that the GPU tests are about, and for BF16 no second fetch of large weights that one feature tile
-would spare."""
+"""The tiles that prompt projections are launched with (csrc/prompt_choice.hpp: the shape chosen and, for int4, where its operands
+stand): those that the GPU tests are about, every depth of the rings that int4 blocks of two token tiles get among them, and for
+BF16 gate and up projections no second fetch of large weights that one feature tile would spare."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -8,14 +8,29 @@ from pathlib import Path
 import pytest
 
 from test_prompt_gated_gpu import GATED
+from test_prompt_tiles_gpu import BLOCKS
 
 ROOT = Path(__file__).resolve().parents[1]
 PROGRAM = r"""
 #include <cstdio>
 #include <cstdlib>
+#include <set>
+#include <tuple>
 #include "prompt_choice.hpp"
 using namespace ei;
-int main(int, char** argv) {
+// Rings and places of the operands of every int4 block of two token tiles.
+int rings() {
+  std::set<std::tuple<int, int, int, int>> seen;
+  for (int n = 144; n <= 40000; n += 272)
+    for (int rows = 33; rows <= 2048; rows += 3) {
+      const PromptTile t = prompt_tensor_operands(PromptShapes(true, rows, n, 896, 148).best(1, false, false).tile);
+      if (t.token_tiles == 2) seen.insert({t.x_stages, t.w_stages, t.raw_stages, int(t.tensor_operands)});
+    }
+  for (const auto& [x, w, raw, tensor] : seen) std::printf("%d %d %d %d ", x, w, raw, tensor);
+  return 0;
+}
+int main(int argc, char** argv) {
+  if (argc == 1) return rings();
   // awq rows features inputs gated -> the tile, its rings and the groups of tokens
   int v[5];
   for (int i = 0; i < 5; ++i) v[i] = std::atoi(argv[1 + i]);
@@ -47,6 +62,15 @@ def launched(tmp_path_factory):
 @pytest.mark.parametrize("awq,rows,hidden,ffn,block", GATED)
 def test_gated_blocks(launched, awq, rows, hidden, ffn, block):
     assert launched(awq, rows, 2 * ffn, hidden, 1)[:7] == block
+
+
+def test_int4_blocks_of_two_token_tiles(launched):
+    """In the order of the GPU test's int4 blocks: the rings they are launched with, and no others exist."""
+    expected = [(3, 2, 2, 0), (3, 2, 4, 1), (3, 3, 6, 1), (4, 4, 8, 1), (4, 4, 8, 1), (5, 4, 8, 1)]
+    blocks = [b for b in BLOCKS if b[0] and not b[4]]
+    assert [launched(1, rows, n, k, 0)[3:7] for _, rows, n, k, _, _ in blocks] == expected
+    every = launched()
+    assert {every[i:i + 4] for i in range(0, len(every), 4)} == set(expected)
 
 
 @pytest.mark.parametrize("rows", [257, 290, 320, 333, 400])

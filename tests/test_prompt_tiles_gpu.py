@@ -62,8 +62,9 @@ def test_awq_tiles(cuda, package, rows, nk):
 
 
 # awq, rows, features, inputs, K slices that the scratch has room for -> feature tiles, token tiles, columns, stages of
-# activations, weight operands and packed weights, K slices (tests/test_prompt_choice_cpu.py holds the shapes to it). 896 inputs
-# are 14 K blocks, which no ring here divides evenly into whole rounds of 3 or 4; every count of rows leaves the last token
+# activations, weight operands and packed weights, K slices (tests/test_prompt_choice_cpu.py holds the shapes to it; int4 is
+# launched with deeper rings where its operands stand in tensor memory: tests/test_prompt_launched_cpu.py). 896 inputs
+# are 14 K blocks, which no ring here divides evenly into whole rounds of 3, 4 or 5; every count of rows leaves the last token
 # tile ragged, and every width the last feature tile.
 BLOCKS = [
     (0, 970, 6256, 896, 0, (1, 2, 176, 3, 3, 0, 1)),
