@@ -11,7 +11,7 @@
 //  * query rows of all heads of a KV group are stacked over the whole row range and dealt to blocks of up to four
 //    warps, 16 stacked rows per warp, so any group size and row count works;
 //  * kernels are compiled for sizes up to 64, 128 and 256, and for keys up to 256 with values up to 128, with the sizes
-//    known at compile time when they are exactly 64, 128 or 192 and 128 (the latter two's prompts: prompt_attention.cuh);
+//    known at compile time when they are exactly 64, 128 or 192 and 128;
 //  * a key may end in a part that all heads share (latent attention's rotated key), fetched from a tensor of its own;
 //  * the finished output may pass a sigmoid gate.
 #include "layered_device.cuh"
@@ -465,7 +465,6 @@ bool launch_tcgen05(const SizedAttentionParams& given, cudaStream_t stream, bool
 
 template <int kKeys, int kValues, bool kExact>
 void launch_bucket(const SizedAttentionParams& p, bool direct, cudaStream_t stream, bool pdl) {
-  constexpr bool kPrompts = !kExact || kKeys == 64;  // of the other exact sizes prompts have a kernel of their own
   static thread_local int configured_device = -1;
   int device = 0;
   EI_CUDA(cudaGetDevice(&device));
@@ -473,20 +472,19 @@ void launch_bucket(const SizedAttentionParams& p, bool direct, cudaStream_t stre
     const int bytes = int(sized_shared_bytes(stages_for(kKeys, kValues), kKeys, kValues));
     EI_CUDA(cudaFuncSetAttribute(sized_attention_kernel<kKeys, kValues, kExact, false>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if constexpr (kPrompts)
-      EI_CUDA(cudaFuncSetAttribute(sized_attention_kernel<kKeys, kValues, kExact, true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    EI_CUDA(cudaFuncSetAttribute(sized_attention_kernel<kKeys, kValues, kExact, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     configured_device = device;
   }
   const int stacked = p.rows * (p.heads / p.kv_heads);
   const int warps = std::min(kMaxWarps, (stacked + 15) / 16);
   const unsigned parts = unsigned((stacked + warps * 16 - 1) / (warps * 16));
   const size_t smem = sized_shared_bytes(stages_for(kKeys, kValues), p.dim_pad, p.vdim_pad);
-  if (!direct)
+  if (direct)
+    launch(sized_attention_kernel<kKeys, kValues, kExact, true>, dim3(p.kv_heads, parts), dim3(warps * 32), smem, stream, pdl, p);
+  else
     launch(sized_attention_kernel<kKeys, kValues, kExact, false>, dim3(p.kv_heads, p.max_splits, parts), dim3(warps * 32), smem,
            stream, pdl, p);
-  else if constexpr (kPrompts)
-    launch(sized_attention_kernel<kKeys, kValues, kExact, true>, dim3(p.kv_heads, parts), dim3(warps * 32), smem, stream, pdl, p);
 }
 
 void launch_sized(const SizedAttentionParams& given, bool direct, cudaStream_t stream, bool pdl) {
@@ -507,13 +505,12 @@ void launch_sized(const SizedAttentionParams& given, bool direct, cudaStream_t s
     if (same && widest == 64) return launch_bucket<64, 64, true>(p, direct, stream, pdl);
     return launch_bucket<64, 64, false>(p, direct, stream, pdl);
   }
-  // Prompts of 128 / 128 and 192 / 128 come here only with a scale that is not positive or queries off 16 bytes.
   if (widest <= 128) {
-    if (same && widest == 128 && !direct) return launch_bucket<128, 128, true>(p, direct, stream, pdl);
+    if (same && widest == 128) return launch_bucket<128, 128, true>(p, direct, stream, pdl);
     return launch_bucket<128, 128, false>(p, direct, stream, pdl);
   }
   if (p.vdim_pad <= 128) {
-    if (p.dim_pad == 192 && p.vdim_pad == 128 && p.k_shift == 3 && !direct) return launch_bucket<192, 128, true>(p, direct, stream, pdl);
+    if (p.dim_pad == 192 && p.vdim_pad == 128 && p.k_shift == 3) return launch_bucket<192, 128, true>(p, direct, stream, pdl);
     return launch_bucket<256, 128, false>(p, direct, stream, pdl);
   }
   return launch_bucket<256, 256, false>(p, direct, stream, pdl);

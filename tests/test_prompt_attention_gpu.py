@@ -169,26 +169,3 @@ def test_a_weight_that_dominates_is_not_rounded(cuda, package):
     got *= np.sqrt((16 * half + (expected ** 2).sum()) / hidden + 1e-6)
     share = (got * expected).sum(-1) / (expected ** 2).sum(-1)
     assert np.abs(share - 1).max() <= 1.9e-3, np.abs(share - 1).max(0)
-
-
-@pytest.mark.parametrize("scale", [-0.08, 0.0])
-def test_scales_that_turn_or_lose_the_scores_order(cuda, package, scale):
-    """Sizes that the tensor-core kernel takes, with scales that it does not: a row's largest score is not its largest exponent."""
-    c = layered_cases.config(64, 64, [layered_cases.parallel((4, 2, 128, 128, 32, 1e5), (1, 16, 16))])
-    c["layers"][0]["mixer"]["left"]["scale"] = scale
-    weights = layered_cases.random_weights(package, c, 8)
-    model = package.Model(*package.checkpoint.admit(c, weights, "zofesun_bf16"))
-    ids = layered_cases.tokens(c, 150)
-    session = model.new_session(160)
-    check_layered(layered_cases.run_portions(session, ids, [100, 50]), hybrid.HybridOracle(c, weights).forward(ids), "bf16")
-
-
-@pytest.mark.parametrize("scale", [-0.06, 0.0])
-def test_latent_scales_that_turn_or_lose_the_scores_order(cuda, package, scale):
-    c = gikepel_cases.config(64, 64, [gikepel_cases.latent(4, 128, 64, 128, 64)])
-    c["layers"][0]["mixer"]["scale"] = scale
-    weights = gikepel_cases.random_weights(package, c, 9)
-    model = package.Model(*package.checkpoint.admit(c, weights, "gikepel_bf16"))
-    ids = layered_cases.tokens(c, 150)
-    session = model.new_session(160)
-    check_gikepel(layered_cases.run_portions(session, ids, [100, 50]), gikepel.GikepelOracle(c, weights).forward(ids), "bf16")
