@@ -1351,7 +1351,8 @@ static void enqueue_mixer_segment(ei_session& s, const LayeredModel::Layer& l, c
     case EI_MIXER_PARALLEL: {
       tick(s);
       launch_mixer_prepare<bf16>(prepare_params(s, l, r, b, false), s.stream, pdl);
-      const SizedAttentionParams a = attention_params(s, l, r, b);
+      SizedAttentionParams a = attention_params(s, l, r, b);
+      a.length = int(context) + rows;
       tick(s);
       launch_sized_attention_prompt(a, s.stream, pdl);
       tick(s);
@@ -1390,6 +1391,7 @@ static void enqueue_mixer_segment(ei_session& s, const LayeredModel::Layer& l, c
       a.out_scale = 1.0f;
       a.device_offset = &s.control->context;
       a.capacity = int(s.capacity);
+      a.length = tokens;
       a.out = b.mixed;
       a.out_stride = l.out.in;
       a.status = &s.control->status;

@@ -141,6 +141,7 @@ struct SizedAttentionParams {
   const float* sink;        // [heads]: exp(sink) joins the denominator; or null
   const int32_t* device_offset;
   int capacity;
+  int length;               // prompt form: tokens up to the segment's end, as the host knows them
   int chunk, max_splits;    // step form
   float* scratch;           // [max_splits][rows * heads][vdim_pad + 4]
   void* out;                // row r, head h at out + r * out_stride + h * vdim_pad

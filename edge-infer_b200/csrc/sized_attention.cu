@@ -441,12 +441,17 @@ void encode_head_map(CUtensorMap* map, const void* base, int tokens, int token_s
 }
 
 // The tcgen05 form: keys in whole 128-byte pieces, rows whose 16-byte pieces can be loaded at once, and a scale that
-// keeps the order of the scores.
+// keeps the order of the scores. Its blocks take a few microseconds more to start and to leave than those of mma.sync, which
+// pays beyond this many tiles of history. Whole prompts, mma.sync against it: 16 heads of 128 / 128 behind 8 (14 such layers,
+// widths 1024 and 2048): 64 rows -3.4 and -2.8 %, 192 -0.4 and +0.3 %, 224 rows behind 192 +2.6 and +4.1 %, 1024 rows +12 and
+// +7 %; 16 of 192 / 128 behind 16 (9 layers): 128 rows -5.2 and -3.3 %, 384 -1.1 and -0.9 %, 33 rows behind 384 +1.4 and
+// +1.7 %, 256 behind 512 +4.8 and +3.7 %.
+constexpr int tcgen05_beyond(int keys) { return (keys == 128 ? 3 : 6) * kTile; }
 template <int kKeys>
 bool launch_tcgen05(const SizedAttentionParams& given, cudaStream_t stream, bool pdl) {
   SizedAttentionParams p = given;
   if (p.dim_pad != kKeys || p.vdim_pad != 128 || p.k_shift != 3 || p.v_shift != 3 || p.q_stride % 8 ||
-      (reinterpret_cast<uintptr_t>(p.q) & 15) || !(p.scale > 0.0f))
+      (reinterpret_cast<uintptr_t>(p.q) & 15) || !(p.scale > 0.0f) || p.length <= tcgen05_beyond(kKeys))
     return false;
   static thread_local int configured_device = -1;
   int device = 0;
