@@ -25,6 +25,18 @@ inline void check_cuda(cudaError_t status, const char* what) {
 }
 #define EI_CUDA(call) ::ei::check_cuda((call), #call)
 
+// Multiprocessors of the current device.
+inline int device_multiprocessors() {
+  static thread_local int known_device = -1, value = 1;
+  int device = 0;
+  EI_CUDA(cudaGetDevice(&device));
+  if (device != known_device) {
+    EI_CUDA(cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device));
+    known_device = device;
+  }
+  return value;
+}
+
 inline void check_launch() { check_cuda(cudaGetLastError(), "kernel launch"); }
 
 using bf16 = __nv_bfloat16;

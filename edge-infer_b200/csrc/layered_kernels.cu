@@ -86,9 +86,10 @@ __global__ void __launch_bounds__(kJoinThreads) sublayer_join_kernel(const Subla
   }
 }
 
-// A unit is 256 bytes a row: a warp that takes one has a single load in flight and waits for it. A prompt's warps take four rows
-// of a unit (1500 rows of 80 units: the whole prompt 7.57 -> 7.44 ms, 14 launches), a step's up to 16 rows one each, so that
-// they fill the chip.
+// A unit is 256 bytes a row: a warp that takes one has a single load in flight and waits for it. Where that would be more than two
+// waves of warps (64 an SM) they take four rows of a unit (1500 rows of 80 units: the whole prompt 7.57 -> 7.44 ms, 14 launches).
+// Fewer rows fill the chip better one each: prompts of 64 rows of 56 units 1.548 -> 1.538 ms, 200 rows 1.758 -> 1.754; the lines
+// meet at about 300 rows of 56 units and 220 of 80.
 // One warp per (kRows rows, unit); units in the order of the fused projection: q heads, k heads, v heads, then the linear
 // attention's q, k and v heads.
 template <typename T, int kRows>
@@ -556,7 +557,7 @@ void launch_sublayer_join(const SublayerJoinParams& p, cudaStream_t stream, bool
 template <typename T>
 void launch_mixer_prepare(const MixerPrepareParams& p, cudaStream_t stream, bool pdl) {
   const int units = p.heads + 2 * p.kv_heads + 3 * p.lin_heads;
-  if (p.rows > kMaxRows)
+  if (p.rows > kMaxRows && p.rows * units > 2 * 64 * device_multiprocessors())
     launch(mixer_prepare_kernel<T, 4>, dim3(unsigned(((p.rows + 3) / 4 * units + 3) / 4)), dim3(128), 0, stream, pdl, p);
   else
     launch(mixer_prepare_kernel<T, 1>, dim3(unsigned((p.rows * units + 3) / 4)), dim3(128), 0, stream, pdl, p);

@@ -106,16 +106,6 @@ inline bool encode_query_map(CUtensorMap* map, const void* q, int rows, int stri
 }
 // Query tiles a block takes: two share the keys and values they read, but where two would leave half of the chip idle the
 // steps of one are shorter (two tiles' exponentials share an SM's 16 a cycle).
-inline int device_multiprocessors() {
-  static thread_local int known_device = -1, value = 1;
-  int device = 0;
-  EI_CUDA(cudaGetDevice(&device));
-  if (device != known_device) {
-    EI_CUDA(cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device));
-    known_device = device;
-  }
-  return value;
-}
 inline int pa_query_tiles(int kv_heads, int stacked, int multiprocessors) {
   return kv_heads * ((stacked + 2 * kPaRows - 1) / (2 * kPaRows)) * 2 <= multiprocessors ? 1 : 2;
 }
