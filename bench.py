@@ -429,7 +429,7 @@ def prompt_leg(shape, ms: float) -> dict:
                          "frac": achieved / peak,
                          "peak_source": "measured (sustained)" if peaks else "fallback"},
             "what": "session prefill of the 2048-token prompt, host tokens in, median of 3 calls; projections on "
-                    "tcgen05 (int4 dequantised in shared memory), one attention launch over all rows"}
+                    "tcgen05 (int4 dequantised into tensor memory), one attention launch over all rows"}
 
 
 def run_sessions_leg(package, torch, dist, rank: int, world: int, rounds: int, profile: bool = False):

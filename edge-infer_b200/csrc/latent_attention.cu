@@ -7,8 +7,9 @@
 // split over blocks along the sequence. The scores and the softmax are FP32; the weights enter the product with the
 // latents as two BF16 terms.
 //
-// A prompt segment expands the keys and values of all cached tokens with the prompt GEMM and runs the tile loop of
-// sized_attention.cu over them, with the rotated part fetched from the cache.
+// A prompt segment expands the keys and values of all cached tokens with the prompt GEMM and runs the prompt attention of
+// sized_attention.cu over them (on the 5th-generation tensor cores where keys are 192 and values 128 wide), with the rotated
+// part fetched from the cache.
 #include "layered_device.cuh"
 
 #include <algorithm>

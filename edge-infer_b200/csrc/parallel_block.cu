@@ -8,8 +8,9 @@ namespace ei {
 namespace {
 
 // Quads of a row that a thread keeps in registers (the rest is read again): four in the blocks of 256 that many rows get, one in
-// a step's blocks of up to 512 or 1024, which have a thread for every quad. (One kernel for all, of 64 registers a thread and
-// four quads, spilled 220 bytes: 2048 rows through 28 layers 10.16 -> 10.07 ms, a step at width 1024 864 -> 856 us.)
+// a step's blocks of up to 512 or 1024, which have a thread for every quad. One kernel for all, of 64 registers a thread and
+// four quads, spilled 220 bytes; these spill nothing but for the join of 1024 threads (92 bytes). 2048 rows through 28 layers
+// 10.16 -> 10.07 ms; steps 1 to 6 % (widths 1024 and 2048: 864 -> 850 and 1326 -> 1246 us a token).
 constexpr int kMostThreads = 1024, kStepThreads = 512, kManyRowThreads = 256;
 constexpr int held_quads(int threads) { return threads == kManyRowThreads ? 4 : 1; }
 

@@ -10,11 +10,17 @@
 // Roles of the twelve warps: 0-3 and 4-7 the softmax of one query tile each (a warp reads the 32 lanes of tensor memory that
 // its place in the four allows), 8 the TMA copies, 9 and 10 the MMAs of one query tile each, 11 the tensor memory.
 //
-// What bounds it: the exponentials (16 a cycle and SM: 1024 cycles for 256 x 64) beside some 1100 cycles of MMAs. On mma.sync,
-// where a tile's MMAs take their scheduler's issue slots, 2048 rows of 32 heads behind 8 KV heads took 129 us a layer; the
-// heaviest of these blocks takes 84 thousand cycles, some 45 us. Whole prompts, before -> now: that shape (36 layers, int4)
-// 33.0 -> 30.7 ms; 333 rows of 16 heads behind 8 (28 layers) 2.39 -> 2.32 ms; 1500 rows of 24 behind 8 (14 layers of 128 / 128
-// wide heads) 8.30 -> 8.00 ms; 2048 rows of 16 heads of 192 / 128 (9 layers) 10.43 -> 10.15 ms.
+// The plan is the published one of attention on this generation of tensor cores (FlashAttention-3, arXiv 2407.08608: two query tiles
+// whose softmax take turns; FlashAttention-4: weights back through tensor memory, outputs rescaled only beyond a slack).
+//
+// What bounds it: the chain scores, softmax, product of each query tile, of which two share an SM. 2048 rows of 32 heads behind 8
+// KV heads, counters of one launch: tensor pipe 42 % of the SM's active cycles, special functions 32 %, issue slots 47 %, 95
+// thousand cycles for the 32 tiles of the longest blocks, some 2900 a tile (where 256 x 64 exponentials at 16 a cycle are 1024 and
+// the MMAs 1100). On mma.sync, where a tile's MMAs take their scheduler's issue slots, that layer took 129 us; it takes 60. Whole
+// prompts, mma.sync -> this (weights relative to a lagging maximum then): that shape (36 layers, int4) 33.0 -> 30.7 ms; 333 rows
+// of 16 heads behind 8 (28 layers) 2.39 -> 2.32; 1500 rows of 16 behind 8 (14 layers of 128 / 128 wide heads) 8.30 -> 8.00; 2048
+// rows of 16 heads of 192 / 128 (9 layers) 10.43 -> 10.15. A block costs some 4 to 5 us to start and to leave, so that short
+// prompts of the layered designs stay on mma.sync (sized_attention.cu).
 //
 // kKeys: 128 or 192 values a key. kSplit: weights keep 16 significant bits, as two BF16 terms, one product each.
 //

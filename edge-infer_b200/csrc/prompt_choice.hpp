@@ -158,7 +158,8 @@ class PromptShapes {
   // (520), 128 x 256 721 (800), 128 x 320 1005-1050 (1056), 128 x 416 1226 (1248)), and launches with FP32 sums come out up
   // to a quarter above their time. Over 332 sizes with every shape and split timed, the one chosen here takes 2.5 % longer
   // than the best in the geometric mean, 27 % at most (int4 3584 x 3584 at 512 rows, 25.8 us for 20.3). Constants fitted to
-  // those times leave 1.5 %.
+  // those times leave 1.5 %. The int4 times are of the kernel with its operands in shared memory, and so are the charges: tiles of
+  // up to 448 tokens, whose operands stand in tensor memory now, are cheaper than this says and 480 tokens are not.
   void add(const PromptTile& t) {
     const int tokens = t.token_tiles * t.columns, mmas = t.feature_tiles * t.token_tiles * (kPromptBlockK / 16);
     const double operand = t.feature_tiles * double(awq_ ? kPromptRawBytes : kPromptWeightBytes);

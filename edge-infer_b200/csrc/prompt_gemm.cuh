@@ -24,7 +24,7 @@
 //     stores have completed. Shared memory is what a K block of many tokens is bound by (activations in, operands out): an
 //     operand in shared memory cost 128 cycles of stores (twice that while rows r and r + 4 met in a bank) and 32 a MMA of
 //     loads. 8B int4, 2048 rows: 30.4 ms with the conflict, 29.2 without, 28.5 from tensor memory; batches of 64 x 5 rows, 7B
-//     int4: 9.45, 9.40, 9.24;
+//     int4: 9.45, 9.40, 9.24 (each row of figures in turn on one GPU; the batch takes 9.2 to 9.9 ms from GPU to GPU);
 //   * one warp or, with more than one accumulator, two (warps 17 and 18) issue, per K block, feature tile and token
 //     tile, four tcgen05.mma (M 128, N columns, K 16) that accumulate in tensor memory, and commit the K block's `empty`
 //     barrier, which hands both operands' buffers back;
@@ -37,14 +37,15 @@
 // issues the MMAs. With one lane walking the issuing loop a K block of a 128-feature tile took 575 (BF16) and 800 (int4)
 // cycles at any number of tokens; with warp-uniform descriptors, one barrier and one commit per K block it takes 380 and
 // 540-560 at up to 160 tokens. Above that it grows with the tile (int4 721 at 256 columns, 1005-1050 at 320, 1226 at 416,
-// counted at 1.9 GHz), and launches that fill the chip run at the rate its power sustains: 320 rows of 37888 x 3584 in
-// 65-68 us, where the sustained cuBLAS rate gives 65. Measured, int4, per launch, first form (tiles of 128 tokens as M, 256
+// counted at 1.9 GHz while the operands stood in shared memory), and launches that fill the chip run at the rate its power
+// sustains: 320 rows of 37888 x 3584 in 64-68 us, where the sustained cuBLAS rate gives 62-65. Measured, int4, per launch, first form (tiles of 128 tokens as M, 256
 // features) -> this one: 37888 x 3584, 320 rows 105 -> 66 us; 24576 x 4096, 2048 rows 344-357 -> 297-331 us (over GPUs);
 // BF16: 4096 x 2048, 333 rows 15 -> 9.9 us.
 // kGated: the gate and up projection of a feed-forward, whose gated units are all that leaves. Their own kernel cost a launch
 // and the pairs' way out and back (6 us at 333 x 12288, 25-37 us at 2048 x 24576); in the epilogue, which nothing overlaps, the
-// units take 23 us of the latter's 305. Whole prompts, separate -> here: 1.7B, 333 rows 2.31 -> 2.18 ms; 8B int4, 2048 rows
-// 30.8 -> 30.5; 1500 rows of the 2048-wide join decoder 8.02 -> 7.67; a batch of 64 x 5 rows, 7B int4 9.80 -> 9.57.
+// units take some 15 us of the latter's 314 (the projection alone 300). Whole prompts, separate -> here, each in turn on one GPU:
+// 1.7B, 333 rows 2.31 -> 2.18 ms; 8B int4, 2048 rows 30.8 -> 30.5; 1500 rows of the 2048-wide join decoder 8.02 -> 7.67; a batch
+// of 64 x 5 rows, 7B int4 9.80 -> 9.57. prompt_choice.hpp has more sizes, and where BF16 takes half tiles.
 // (An int4 tile of 480 tokens leaves no columns: its operands stand in shared memory, swizzled, K-major, as BF16 ones do.)
 // Rows beyond T and features beyond N are zero-filled by TMA and masked in the epilogue.
 //
